@@ -139,10 +139,23 @@ int copy_field(afid_ctx_t *ctx, double *dst, const double *src, int ld_x, int ld
   return AFID_OK;
 }
 
-int check_err_flag(afid_ctx_t *ctx) {
-  int h = 0;
-  AFID_CUDA(ctx, cudaMemcpyAsync(&h, ctx->err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+// Words 0 .. n-1 of ctx->red to host_scratch, the error word (1) among them, and its status.
+int read_status(afid_ctx_t *ctx, int n) {
+  AFID_CUDA(ctx, cudaMemcpyAsync(ctx->host_scratch, ctx->red, n * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
   AFID_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  int h;
+  std::memcpy(&h, ctx->host_scratch + 1, sizeof(int));
+  if (h & 1) return AFID_E_SINGULAR;
+  if (h & 2) return AFID_E_TIMEOUT;
+  return AFID_OK;
+}
+
+// The status alone; host_scratch[0 .. 6] may hold results of copies issued before.
+int check_err_flag(afid_ctx_t *ctx) {
+  AFID_CUDA(ctx, cudaMemcpyAsync(ctx->host_scratch + 7, ctx->red + 1, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+  AFID_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  int h;
+  std::memcpy(&h, ctx->host_scratch + 7, sizeof(int));
   if (h & 1) return AFID_E_SINGULAR;
   if (h & 2) return AFID_E_TIMEOUT;
   return AFID_OK;
@@ -395,8 +408,8 @@ int ctx_create(const afid_grid_t *grid, const afid_params_t *prm, const BatchSpe
   const size_t nsets = bs ? (size_t)bs->ninst : 1;  // batch mode: one table set per instance
   chk(dalloc(ctx, &ctx->cn_tab, cn_tab_doubles(M, 3) * nsets));
   chk(dalloc(ctx, &ctx->sc, 3 * nsets));
-  chk(dalloc(ctx, &ctx->err, 1));
-  chk(dalloc(ctx, &ctx->red, 1));
+  chk(dalloc(ctx, &ctx->red, 2 * kReduceWords));
+  ctx->err = reinterpret_cast<int *>(ctx->red + 1);
   const int nb = globals_partial_blocks(g);
   chk(dalloc(ctx, &ctx->partial, (size_t)nb * 3));
   chk(dalloc(ctx, &ctx->gsum, 3));
@@ -925,8 +938,7 @@ int afid_gpu_cfl(afid_ctx_t *ctx, double *cflm) {
   cudaSetDevice(ctx->dev);
   AFID_CUDA(ctx, timed(ctx, 8, [&] { return launch_max_reduce(ctx->L, false, ctx->vx, ctx->vy, ctx->vz, ctx->red); }));
   ctx->launches += 1;
-  AFID_CUDA(ctx, cudaMemcpyAsync(ctx->host_scratch, ctx->red, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-  int s = check_err_flag(ctx);
+  const int s = read_status(ctx, 2);
   const double v = ctx->host_scratch[0];
   *cflm = (v != v) ? v : std::max(0.00000001, v);  // CalcMaxCFL.F90:22; a NaN maximum is passed on
   return s;
@@ -937,8 +949,7 @@ int afid_gpu_divmax(afid_ctx_t *ctx, double *dmax) {
   cudaSetDevice(ctx->dev);
   AFID_CUDA(ctx, timed(ctx, 8, [&] { return launch_max_reduce(ctx->L, true, ctx->vx, ctx->vy, ctx->vz, ctx->red); }));
   ctx->launches += 1;
-  AFID_CUDA(ctx, cudaMemcpyAsync(ctx->host_scratch, ctx->red, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-  int s = check_err_flag(ctx);
+  const int s = read_status(ctx, 2);
   *dmax = ctx->host_scratch[0];
   return s;
 }
@@ -1234,8 +1245,9 @@ int afid_gpu_sal_create(afid_ctx_t *ctx, const afid_sal_grid_t *sg) {
     if ((e = up(sts[d]->w, (size_t)4 * sts[d]->n, &st.w[d])) != cudaSuccess) return fail(e);
   }
   if ((e = dalloc(ctx, &S->cn_tab, cn_tab_doubles(MR, 1))) != cudaSuccess ||  // 3 substeps x 1 matrix
-      (e = dalloc(ctx, &S->sc, 3)) != cudaSuccess || (e = dalloc(ctx, &S->red, 1)) != cudaSuccess)
+      (e = dalloc(ctx, &S->sc, 3)) != cudaSuccess)
     return fail(e);
+  S->red = ctx->red + kReduceWords;
   S->prof_blocks = sal_prof_blocks(q);
   if ((e = dalloc(ctx, &S->partial, (size_t)S->prof_blocks * 6 * nxmr)) != cudaSuccess ||
       (e = dalloc(ctx, &S->prof_out, (size_t)6 * nxmr)) != cudaSuccess)
@@ -1282,10 +1294,8 @@ int afid_gpu_sal_cfl(afid_ctx_t *ctx, double *cflmr) {
   cudaSetDevice(ctx->dev);
   AFID_CUDA(ctx, timed(ctx, 8, [&] { return launch_sal_cfl(ctx->L, *ctx->sal); }));
   ctx->launches += 1;
-  AFID_CUDA(ctx, cudaMemcpyAsync(ctx->host_scratch, ctx->sal->red, sizeof(double), cudaMemcpyDeviceToHost,
-                                 ctx->stream));
-  const int s = check_err_flag(ctx);
-  const double v = ctx->host_scratch[0];
+  const int s = read_status(ctx, kReduceWords + 1);
+  const double v = ctx->host_scratch[kReduceWords];
   *cflmr = (v != v) ? v : std::max(1.0e-8, v);  // CalcMaxCFL.F90:50; a NaN maximum is passed on
   return s;
 }

@@ -6,6 +6,7 @@
 // instance on the device, so one step is a fixed launch sequence, captured into a CUDA graph.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <new>
@@ -28,6 +29,7 @@ struct InstCtl {
 __global__ void __launch_bounds__(256)
     k_batch_cfl(Geom g, Tables t, const double *__restrict__ vx, const double *__restrict__ vy,
                 const double *__restrict__ vz, unsigned long long *__restrict__ out) {
+  chain_begin();
   const int i = blockIdx.y;
   if (!inst_active(g, i)) return;
   bind_instance(g, i);
@@ -72,15 +74,18 @@ __global__ void __launch_bounds__(256)
 // dt rule of main.F90:287-304 per instance.  An instance whose previous step raised an error
 // code is switched off before this step (the reference exits after the step that set it).
 __global__ void k_batch_dt(int nslots, unsigned char *__restrict__ active, const InstCtl *__restrict__ ctl,
-                           const unsigned long long *__restrict__ cfl_bits, const int *__restrict__ ntime,
+                           unsigned long long *__restrict__ cfl_bits, const int *__restrict__ ntime,
                            double *__restrict__ dt, double *__restrict__ cfl, int *__restrict__ err) {
+  chain_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nslots || !active[i]) return;
+  const unsigned long long bits = cfl_bits[i];
+  cfl_bits[i] = 0;  // the next step's maximum starts here
   if (err[i] != 0) {
     active[i] = 0;
     return;
   }
-  const double cflm = nan_max(0.00000001, __longlong_as_double((long long)cfl_bits[i]));  // CalcMaxCFL.F90:22
+  const double cflm = nan_max(0.00000001, __longlong_as_double((long long)bits));  // CalcMaxCFL.F90:22
   const InstCtl c = ctl[i];
   double d = dt[i];
   if (c.idtv == 1) {
@@ -100,6 +105,7 @@ __global__ void k_batch_dt(int nslots, unsigned char *__restrict__ active, const
 // time += dt (main.F90:313), step counter; a slot that reached its step limit switches off.
 __global__ void k_batch_advance(int nslots, unsigned char *__restrict__ active, const double *__restrict__ dt,
                                 double *__restrict__ time, int *__restrict__ ntime, const int *__restrict__ limit) {
+  chain_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nslots || !active[i]) return;
   time[i] += dt[i];
@@ -270,23 +276,21 @@ int reset_slot(afid_batch_t *b, int slot) {
 int enqueue_step(afid_batch_t *b) {
   afid_ctx_t *ctx = b->ctx;
   const LaunchCtx &L = ctx->L;
-  cudaStream_t st = ctx->stream;
   if (b->three_d) {
     if (launch_max_reduce(L, false, ctx->vx, ctx->vy, ctx->vz, b->cfl_bits) != cudaSuccess) return AFID_E_CUDA;
   } else {
-    if (cudaMemsetAsync(b->cfl_bits, 0, sizeof(unsigned long long) * b->nslots, st) != cudaSuccess)
-      return AFID_E_CUDA;
-    k_batch_cfl<<<dim3(kChunks, b->nslots), 256, 0, st>>>(L.g, L.t, ctx->vx, ctx->vy, ctx->vz, b->cfl_bits);
+    launch_chained(L, k_batch_cfl, dim3(kChunks, b->nslots), 256, 0, L.g, L.t, ctx->vx, ctx->vy,
+                   ctx->vz, b->cfl_bits);
   }
-  k_batch_dt<<<(b->nslots + 127) / 128, 128, 0, st>>>(b->nslots, ctx->active_dev, b->ctl, b->cfl_bits, b->ntime,
-                                                      b->dt, b->cfl, b->err);
+  launch_chained(L, k_batch_dt, (b->nslots + 127) / 128, 128, 0, b->nslots, ctx->active_dev, b->ctl, b->cfl_bits,
+                 b->ntime, b->dt, b->cfl, b->err);
   ctx->launches += 3;  // with k_batch_advance below
   if (cudaGetLastError() != cudaSuccess) return AFID_E_CUDA;
   int s = ctx_build_cn_batch(ctx, b->dt);
   for (int ns = 0; s == AFID_OK && ns < ctx->nsst; ++ns) s = ctx_run_substep(ctx, ns);
   if (s != AFID_OK) return s;
-  k_batch_advance<<<(b->nslots + 127) / 128, 128, 0, st>>>(b->nslots, ctx->active_dev, b->dt, b->time, b->ntime,
-                                                           b->limit);
+  launch_chained(L, k_batch_advance, (b->nslots + 127) / 128, 128, 0, b->nslots, ctx->active_dev, b->dt, b->time,
+                 b->ntime, b->limit);
   return cudaGetLastError() == cudaSuccess ? AFID_OK : AFID_E_CUDA;
 }
 
@@ -405,7 +409,7 @@ int afid_batch_create(const afid_input_t *proto, int nslots, int precision, afid
   chk(balloc(b, &b->ntime, nslots));
   chk(balloc(b, &b->err, nslots));
   chk(balloc(b, &b->limit, nslots));
-  chk(balloc(b, &b->cfl_bits, nslots));
+  chk(balloc(b, &b->cfl_bits, std::max(nslots, kReduceWords)));
   chk(balloc(b, &b->partial, (size_t)nslots * kChunks * 3));
   chk(balloc(b, &b->gsum, (size_t)nslots * 3));
   if (e == cudaSuccess) e = cudaMallocHost(&b->host, (size_t)nslots * 8 * sizeof(double));
@@ -551,7 +555,9 @@ int afid_batch_step(afid_batch_t *b, int nsteps) {
       cudaGraph_t graph = nullptr;
       cudaError_t e = cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal);
       if (e != cudaSuccess) return ctx_fail(ctx, e);
+      ctx->L.chained = false;  // see launch_chained
       int s = enqueue_step(b);
+      ctx->L.chained = true;
       e = cudaStreamEndCapture(ctx->stream, &graph);
       ctx->temp = temp0;
       ctx->temp_o = tempo0;
@@ -670,6 +676,8 @@ int afid_batch_divmax(afid_batch_t *b, double *dmax) {
   std::vector<unsigned long long> h(b->nslots);
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(h.data(), b->cfl_bits, sizeof(unsigned long long) * b->nslots, cudaMemcpyDeviceToHost, st);
+  if (e == cudaSuccess && !b->three_d)  // the step control's maxima start from zero
+    e = cudaMemsetAsync(b->cfl_bits, 0, sizeof(unsigned long long) * b->nslots, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) return ctx_fail(ctx, e);
   for (int i = 0; i < b->nslots; ++i) {

@@ -14,6 +14,16 @@
 namespace afid {
 
 constexpr int kWarp = 32;
+
+// First statement of every kernel that launch_chained (afid_internal.h) starts: such a kernel may
+// be scheduled while the previous one of its stream still runs.  The wait holds every thread until
+// that kernel has completed and its writes are visible; a kernel of the chain therefore cannot
+// complete before all earlier ones.  Then the next kernel may be scheduled in turn: its launch
+// latency (about 2 us between dependent kernels) passes while this one runs.
+__device__ __forceinline__ void chain_begin() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
 constexpr int kMaxFftPasses = 24;
 
 struct Geom {
@@ -470,6 +480,18 @@ constexpr long long kDrainLimit = 1LL << 28;
 // Maximum that propagates NaN (fmax drops it): a NaN anywhere in a CFL or divergence
 // reduction makes the result NaN, which the main-loop checks turn into an error code.
 __device__ __forceinline__ double nan_max(double a, double b) { return (b > a || b != b) ? b : a; }
+
+// The block maxima of a reduction kernel into out[0] (bit pattern of a non-negative double, or of
+// a NaN, which is larger), by one thread a block.  out[2] accumulates and out[3] counts the blocks;
+// the last block hands the maximum over and leaves both at zero for the next launch, so no
+// memset has to precede it.
+__device__ __forceinline__ void reduce_publish(unsigned long long *out, double v) {
+  atomicMax(out + 2, (unsigned long long)__double_as_longlong(v));
+  __threadfence();
+  if (atomicInc(reinterpret_cast<unsigned int *>(out + 3), gridDim.x - 1) == gridDim.x - 1)
+    out[0] = atomicExch(out + 2, 0ULL);
+}
+constexpr int kReduceWords = 4;  // out[0] result, out[1] not touched, out[2] and out[3] as above
 
 // 1-D TMA bulk copies global -> shared, completed on an mbarrier (sm_90+ PTX, no tensor map,
 // no multicast).  Source and destination must be 16-byte aligned, size a multiple of 16.

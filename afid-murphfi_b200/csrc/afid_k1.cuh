@@ -451,6 +451,7 @@ __global__ void __launch_bounds__(TPC, k1_min_blocks<CAP, TPC>())
                         TE *__restrict__ rux, TE *__restrict__ ruy, TE *__restrict__ ruz,
                         TE *__restrict__ rut, double *__restrict__ vx_o, double *__restrict__ vy_o,
                         double *__restrict__ vz_o, double *__restrict__ temp_o, int *__restrict__ err) {
+  chain_begin();
   constexpr int LD = chunk_ld(M);
   constexpr int FLD = LD * M;
   constexpr int H = POL & 1;  // cache policy of the global loads (tld / nld / sld above)
@@ -695,6 +696,7 @@ __global__ void __launch_bounds__(TPC, k1_min_blocks<CAP, TPC>())
                            TE *__restrict__ rux, TE *__restrict__ ruy, TE *__restrict__ ruz,
                            TE *__restrict__ rut, double *__restrict__ vx_o, double *__restrict__ vy_o,
                            double *__restrict__ vz_o, double *__restrict__ temp_o, int *__restrict__ err) {
+  chain_begin();
   constexpr int LD = chunk_ld(M);
   constexpr int FLD = LD * M;
   constexpr int H = POL & 1;
@@ -941,9 +943,8 @@ cudaError_t launch_k1y2_cfg(const LaunchCtx &L, const SubstepBuffers &b, int ns,
   auto kern = k_explicit_implicit_y2<M, TPC, RPT, TE, TWO_D, CAP, SAL, POL>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  kern<<<ncol / 2, TPC, smem, L.stream>>>(L.g, L.t, b.sc, ns, b.cn_tab, b.vx, b.vy, b.vz, b.temp, b.pr,
-                                          (TE *)b.rux, (TE *)b.ruy, (TE *)b.ruz, (TE *)b.rut, b.vx_o, b.vy_o,
-                                          b.vz_o, b.temp_o, b.err);
+  launch_chained(L, kern, ncol / 2, TPC, smem, L.g, L.t, b.sc, ns, b.cn_tab, b.vx, b.vy, b.vz, b.temp, b.pr,
+                 (TE *)b.rux, (TE *)b.ruy, (TE *)b.ruz, (TE *)b.rut, b.vx_o, b.vy_o, b.vz_o, b.temp_o, b.err);
   return cudaGetLastError();
 }
 
@@ -999,6 +1000,7 @@ __global__ void __launch_bounds__(TPC * G, 1)
                           TE *__restrict__ rut, double *__restrict__ vx_o, double *__restrict__ vy_o,
                           double *__restrict__ vz_o, double *__restrict__ temp_o, int *__restrict__ err,
                           int ncol) {
+  chain_begin();
   constexpr int LD = chunk_ld(M);
   constexpr int FLD = LD * M;
   constexpr int CS = k1_col_stride(M);
@@ -1223,9 +1225,8 @@ cudaError_t launch_k1p_cfg(const LaunchCtx &L, const SubstepBuffers &b, int ns, 
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     const int grid = std::min(nsm, (ncol + G - 1) / G);
-    kern<<<grid, TPC * G, smem, L.stream>>>(L.g, L.t, b.sc, ns, b.cn_tab, b.vx, b.vy, b.vz, b.temp, b.pr,
-                                            (TE *)b.rux, (TE *)b.ruy, (TE *)b.ruz, (TE *)b.rut, b.vx_o, b.vy_o,
-                                            b.vz_o, b.temp_o, b.err, ncol);
+    launch_chained(L, kern, grid, TPC * G, smem, L.g, L.t, b.sc, ns, b.cn_tab, b.vx, b.vy, b.vz, b.temp, b.pr,
+                   (TE *)b.rux, (TE *)b.ruy, (TE *)b.ruz, (TE *)b.rut, b.vx_o, b.vy_o, b.vz_o, b.temp_o, b.err, ncol);
     return cudaGetLastError();
   }
 }
@@ -1236,9 +1237,8 @@ cudaError_t launch_k1_cfg(const LaunchCtx &L, const SubstepBuffers &b, int ns, i
   auto kern = k_explicit_implicit<M, TPC, RPT, TE, TWO_D, CAP, SAL, POL>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  kern<<<ncol, TPC, smem, L.stream>>>(L.g, L.t, b.sc, ns, b.cn_tab, b.vx, b.vy, b.vz, b.temp, b.pr,
-                                      (TE *)b.rux, (TE *)b.ruy, (TE *)b.ruz, (TE *)b.rut, b.vx_o, b.vy_o,
-                                      b.vz_o, b.temp_o, b.err);
+  launch_chained(L, kern, ncol, TPC, smem, L.g, L.t, b.sc, ns, b.cn_tab, b.vx, b.vy, b.vz, b.temp, b.pr, (TE *)b.rux,
+                 (TE *)b.ruy, (TE *)b.ruz, (TE *)b.rut, b.vx_o, b.vy_o, b.vz_o, b.temp_o, b.err);
   return cudaGetLastError();
 }
 

@@ -65,6 +65,7 @@ struct CnBuildArgs {
 
 __global__ void k_cn_tables(CnBuildArgs args, int M, double *__restrict__ tab,
                             StepCoef *__restrict__ sc) {
+  chain_begin();
   const int lane = threadIdx.x;
   const int m = blockIdx.x % args.nmat;
   const int sub = (blockIdx.x / args.nmat) % args.nsub;
@@ -181,6 +182,7 @@ __global__ void __launch_bounds__(256)
                 const double *__restrict__ vx, const double *__restrict__ vy,
                 const double *__restrict__ vz, typename Cplx<TS>::type *__restrict__ spec,
                 FftPlan pl, const typename Cplx<TS>::type *__restrict__ tw, const double *__restrict__ field) {
+  chain_begin();
   using C = typename Cplx<TS>::type;
   extern __shared__ __align__(16) unsigned char smem_raw_k2[];
   C *b0 = reinterpret_cast<C *>(smem_raw_k2);
@@ -241,6 +243,7 @@ template <int TXZ, bool INV, typename TS>
 __global__ void __launch_bounds__(256)
     k_fft_z(Geom g, typename Cplx<TS>::type *__restrict__ spec, FftPlan pl,
             const typename Cplx<TS>::type *__restrict__ tw) {
+  chain_begin();
   using C = typename Cplx<TS>::type;
   extern __shared__ __align__(16) unsigned char smem_raw_k3[];
   C *b0 = reinterpret_cast<C *>(smem_raw_k3);
@@ -280,6 +283,7 @@ template <int M, int WPB, typename TS>
 __global__ void __launch_bounds__(WPB * 32)
     k_tridiag_pressure(Geom g, Tables t, typename Cplx<TS>::type *__restrict__ spec,
                        int *__restrict__ err) {
+  chain_begin();
   using C = typename Cplx<TS>::type;
   extern __shared__ double smem_k4[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -430,6 +434,7 @@ template <int TX, typename TS>
 __global__ void __launch_bounds__(256)
     k_ifft_y(Geom g, const typename Cplx<TS>::type *__restrict__ spec, TS *__restrict__ phi,
              FftPlan pl, const typename Cplx<TS>::type *__restrict__ tw) {
+  chain_begin();
   using C = typename Cplx<TS>::type;
   extern __shared__ __align__(16) unsigned char smem_raw_k6[];
   C *b0 = reinterpret_cast<C *>(smem_raw_k6);
@@ -491,6 +496,7 @@ __global__ void __launch_bounds__(256)
               const double *__restrict__ vxh, const double *__restrict__ vyh,
               const double *__restrict__ vzh, double *__restrict__ vx, double *__restrict__ vy,
               double *__restrict__ vz, double *__restrict__ pr, const TS *__restrict__ phi) {
+  chain_begin();
   using V = typename Vec2<TS>::type;
   const int k0 = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
@@ -585,6 +591,7 @@ template <bool DIV>
 __global__ void __launch_bounds__(256)
     k_max_reduce(Geom g, Tables t, const double *__restrict__ vx, const double *__restrict__ vy,
                  const double *__restrict__ vz, unsigned long long *__restrict__ out) {
+  chain_begin();
   __shared__ double red[8];
   double m = 0.0;
   const int lane = threadIdx.x & 31;
@@ -613,7 +620,7 @@ __global__ void __launch_bounds__(256)
   if (threadIdx.x < 32) {
     double v = (threadIdx.x < (blockDim.x >> 5)) ? red[threadIdx.x] : 0.0;
     v = warp_max(v);
-    if (threadIdx.x == 0) atomicMax(out, (unsigned long long)__double_as_longlong(v));
+    if (threadIdx.x == 0) reduce_publish(out, v);
   }
 }
 
@@ -693,6 +700,7 @@ __global__ void __launch_bounds__(256)
                   const double *__restrict__ vx, const double *__restrict__ vy,
                   const double *__restrict__ vz, typename Cplx<TS>::type *__restrict__ spec,
                   const typename Cplx<TS>::type *__restrict__ tw, const double *__restrict__ field) {
+  chain_begin();
   using C = typename Cplx<TS>::type;
   constexpr int N = 32 * N1;
   extern __shared__ __align__(16) unsigned char smem_k2w[];
@@ -845,6 +853,7 @@ template <int N1>
 __global__ void __launch_bounds__(256, div_blocks_by_regs<N1>())
     k_div_fft_y_wt(Geom g, Tables t, const StepCoef *__restrict__ sc_all, int ns, const __grid_constant__ DivMaps mp,
                    double2 *__restrict__ spec, const double2 *__restrict__ tw, int *__restrict__ err) {
+  chain_begin();
   constexpr int N = 32 * N1;
   if (!inst_active(g, 0)) return;  // a single domain stopped by its step control
   extern __shared__ __align__(1024) unsigned char smem_k2t[];
@@ -968,6 +977,7 @@ template <int N1, bool INV, typename TS>
 __global__ void __launch_bounds__(256)
     k_fft_z_w(Geom g, typename Cplx<TS>::type *__restrict__ spec,
               const typename Cplx<TS>::type *__restrict__ tw) {
+  chain_begin();
   using C = typename Cplx<TS>::type;
   constexpr int N = 32 * N1;
   extern __shared__ __align__(16) unsigned char smem_k3w[];
@@ -1025,6 +1035,7 @@ template <int N1, bool INV, typename TS>
 __global__ void __launch_bounds__(256)
     k_fft_z_wp(Geom g, typename Cplx<TS>::type *__restrict__ spec,
                const typename Cplx<TS>::type *__restrict__ tw) {
+  chain_begin();
   using C = typename Cplx<TS>::type;
   constexpr int N = 32 * N1;
   extern __shared__ __align__(16) unsigned char smem_k3p[];
@@ -1120,6 +1131,7 @@ template <int N1, bool INV, typename TS>
 __global__ void __launch_bounds__(256)
     k_fft_z_wt(Geom g, const __grid_constant__ CUtensorMap ld_map, const __grid_constant__ CUtensorMap st_map,
                const typename Cplx<TS>::type *__restrict__ tw, int *__restrict__ err) {
+  chain_begin();
   using C = typename Cplx<TS>::type;
   constexpr int N = 32 * N1;
   // a tile row is 128 bytes: 8 x points of double2, or 16 of float2 (two columns a warp)
@@ -1255,6 +1267,7 @@ template <int N1, typename TS>
 __global__ void __launch_bounds__(256)
     k_ifft_y_w(Geom g, const typename Cplx<TS>::type *__restrict__ spec, TS *__restrict__ phi,
                const typename Cplx<TS>::type *__restrict__ tw) {
+  chain_begin();
   using C = typename Cplx<TS>::type;
   constexpr int N = 32 * N1;
   constexpr int NH = N / 2 + 1;
@@ -1338,6 +1351,7 @@ template <int N1>
 __global__ void __launch_bounds__(256)
     k_ifft_y_wt(Geom g, const __grid_constant__ CUtensorMap ld_map, const __grid_constant__ CUtensorMap st_map,
                 const double2 *__restrict__ tw, int *__restrict__ err) {
+  chain_begin();
   constexpr int N = 32 * N1;
   constexpr int NH = N / 2 + 1;
   constexpr int HB = (NH * 128 + 1023) / 1024 * 1024;  // bytes of one staged half, 1024-aligned
@@ -1497,7 +1511,7 @@ cudaError_t launch_cn_tables(const LaunchCtx &L, const CnInputs &in) {
   a.inst = in.inst;
   a.active = in.active;
   const int nb = in.dt_dev ? in.ninst : 1;
-  k_cn_tables<<<in.nmat * in.nsub * nb, 32, 0, L.stream>>>(a, in.M, in.tab, in.sc);
+  launch_chained(L, k_cn_tables, in.nmat * in.nsub * nb, 32, 0, a, in.M, in.tab, in.sc);
   return cudaGetLastError();
 }
 
@@ -1517,6 +1531,7 @@ cudaError_t launch_explicit_implicit(const LaunchCtx &L, const SubstepBuffers &b
 template <int M, int WPB, typename TS>
 __global__ void __launch_bounds__(WPB * 32, (WPB == 4) ? 4 : 2)
     k_tridiag_pressure_p(Geom g, Tables t, typename Cplx<TS>::type *__restrict__ spec, int *__restrict__ err) {
+  chain_begin();
   using C = typename Cplx<TS>::type;
   extern __shared__ double smem_k4p[];
   constexpr int LD = chunk_ld(M);
@@ -1694,7 +1709,7 @@ static cudaError_t launch_k4p_M(const LaunchCtx &L, void *spec, int *err) {
   auto kern = k_tridiag_pressure_p<M, W, TS>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  kern<<<k4p_grid(kern, nsys, W, smem), W * 32, smem, L.stream>>>(L.g, L.t, (typename Cplx<TS>::type *)spec, err);
+  launch_chained(L, kern, k4p_grid(kern, nsys, W, smem), W * 32, smem, L.g, L.t, (typename Cplx<TS>::type *)spec, err);
   return cudaGetLastError();
 }
 
@@ -1705,7 +1720,7 @@ static cudaError_t launch_k4_M(const LaunchCtx &L, void *spec, int *err) {
   const size_t smem = (size_t)W * (M <= 8 ? 5 : 4) * chunk_ld(M) * M * sizeof(double);
   auto kern = k_tridiag_pressure<M, W, TS>;
   cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  kern<<<(nsys + W - 1) / W, W * 32, smem, L.stream>>>(L.g, L.t, (typename Cplx<TS>::type *)spec, err);
+  launch_chained(L, kern, (nsys + W - 1) / W, W * 32, smem, L.g, L.t, (typename Cplx<TS>::type *)spec, err);
   return cudaGetLastError();
 }
 
@@ -1788,15 +1803,15 @@ static cudaError_t launch_w_n1(const LaunchCtx &L, const SubstepBuffers &b, int 
         if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || nsm < 1) nsm = 148;
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, 256, sm2) != cudaSuccess || per < 1) per = 1;
         const int ntiles = ((g.nxm + 15) / 16) * g.nzm;
-        kern<<<std::max(1, std::min(ntiles, nsm * per)), 256, sm2, L.stream>>>(g, L.t, b.sc, ns, mp, spec,
-                                                                              (const double2 *)L.twy, b.err);
+        launch_chained(L, kern, std::max(1, std::min(ntiles, nsm * per)), 256, sm2, g, L.t, b.sc, ns, mp, spec,
+                       (const double2 *)L.twy, b.err);
       }
     } else if (st == Stage::DivFftY) {
       const size_t smt = sm + (lane_table_fits(sm, lane_table_bytes<N1, C>()) ? lane_table_bytes<N1, C>() : 0);
       auto kern = k_div_fft_y_w<N1, TS>;
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smt);
-      kern<<<grid, 256, smt, L.stream>>>(g, L.t, b.sc, ns, b.vx_o, b.vy_o, b.vz_o, spec, (const C *)L.twy,
-                                         b.fft_field);
+      launch_chained(L, kern, grid, 256, smt, g, L.t, b.sc, ns, b.vx_o, b.vy_o, b.vz_o, spec, (const C *)L.twy,
+                     b.fft_field);
     } else if (L.ify_var == 1) {  // tensor copies (FP64 single domain, N <= 384)
       if constexpr (!std::is_same<TS, double>::value || N1 > 12) {
         return cudaErrorInvalidValue;
@@ -1816,8 +1831,8 @@ static cudaError_t launch_w_n1(const LaunchCtx &L, const SubstepBuffers &b, int 
         if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || nsm < 1) nsm = 148;
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, 256, sm6) != cudaSuccess || per < 1) per = 1;
         const int ntiles = ((g.nxm + 15) / 16) * g.nzm;
-        kern<<<std::max(1, std::min(ntiles, nsm * per)), 256, sm6, L.stream>>>(g, ld_map, st_map,
-                                                                              (const double2 *)L.twy, b.err);
+        launch_chained(L, kern, std::max(1, std::min(ntiles, nsm * per)), 256, sm6, g, ld_map, st_map,
+                       (const double2 *)L.twy, b.err);
       }
     } else {
       // the staged half spectrum [N/2 + 1][16] is 16 elements larger than the [N][8] tile
@@ -1825,7 +1840,7 @@ static cudaError_t launch_w_n1(const LaunchCtx &L, const SubstepBuffers &b, int 
       if (lane_table_fits(sm6, lane_table_bytes<N1, C>())) sm6 += lane_table_bytes<N1, C>();
       auto kern = k_ifft_y_w<N1, TS>;
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm6);
-      kern<<<grid, 256, sm6, L.stream>>>(g, spec, (TS *)b.phi, (const C *)L.twy);
+      launch_chained(L, kern, grid, 256, sm6, g, spec, (TS *)b.phi, (const C *)L.twy);
     }
     return cudaGetLastError();
   }
@@ -1846,8 +1861,8 @@ static cudaError_t launch_w_n1(const LaunchCtx &L, const SubstepBuffers &b, int 
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, 256, smb) != cudaSuccess || per < 1) per = 1;
     constexpr int XT = 128 / (int)sizeof(C);  // x points a tile
     const int ntiles = ((g.nxm + XT - 1) / XT) * g.nyh;
-    kern<<<std::max(1, std::min(ntiles, nsm * per)), 256, smb, L.stream>>>(g, ld_map, st_map, (const C *)L.twz,
-                                                                          b.err);
+    launch_chained(L, kern, std::max(1, std::min(ntiles, nsm * per)), 256, smb, g, ld_map, st_map, (const C *)L.twz,
+                   b.err);
     return cudaGetLastError();
   }
   if (L.fftz_var == 1) {  // persistent, double-buffered tiles
@@ -1861,14 +1876,14 @@ static cudaError_t launch_w_n1(const LaunchCtx &L, const SubstepBuffers &b, int 
     if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || nsm < 1) nsm = 148;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, 256, smp) != cudaSuccess || per < 1) per = 1;
     const int ntiles = ((g.nxm + 7) / 8) * g.nyh;
-    kern<<<std::max(1, std::min(ntiles, nsm * per)), 256, smp, L.stream>>>(g, spec, (const C *)L.twz);
+    launch_chained(L, kern, std::max(1, std::min(ntiles, nsm * per)), 256, smp, g, spec, (const C *)L.twz);
     return cudaGetLastError();
   }
   dim3 grid((g.nxm + 7) / 8, g.nyh);
   const size_t smt = sm + (lane_table_fits(sm, lane_table_bytes<N1, C>()) ? lane_table_bytes<N1, C>() : 0);
   auto kern = (st == Stage::FftZFwd) ? k_fft_z_w<N1, false, TS> : k_fft_z_w<N1, true, TS>;
   cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smt);
-  kern<<<grid, 256, smt, L.stream>>>(g, spec, (const C *)L.twz);
+  launch_chained(L, kern, grid, 256, smt, g, spec, (const C *)L.twz);
   return cudaGetLastError();
 }
 
@@ -1911,16 +1926,16 @@ static cudaError_t launch_stage_T(const LaunchCtx &L, const SubstepBuffers &b, i
       dim3 grid((g.nxm + TX - 1) / TX, g.nzm);
       if (TX == 8) {
         cudaFuncSetAttribute(k_div_fft_y<8, TS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        k_div_fft_y<8, TS><<<grid, 256, smem, L.stream>>>(g, L.t, b.sc, ns, b.vx_o, b.vy_o, b.vz_o, spec,
-                                                          L.plan_y, twy, b.fft_field);
+        launch_chained(L, k_div_fft_y<8, TS>, grid, 256, smem, g, L.t, b.sc, ns, b.vx_o, b.vy_o, b.vz_o, spec,
+                       L.plan_y, twy, b.fft_field);
       } else if (TX == 4) {
         cudaFuncSetAttribute(k_div_fft_y<4, TS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        k_div_fft_y<4, TS><<<grid, 256, smem, L.stream>>>(g, L.t, b.sc, ns, b.vx_o, b.vy_o, b.vz_o, spec,
-                                                          L.plan_y, twy, b.fft_field);
+        launch_chained(L, k_div_fft_y<4, TS>, grid, 256, smem, g, L.t, b.sc, ns, b.vx_o, b.vy_o, b.vz_o, spec,
+                       L.plan_y, twy, b.fft_field);
       } else {
         cudaFuncSetAttribute(k_div_fft_y<2, TS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        k_div_fft_y<2, TS><<<grid, 256, smem, L.stream>>>(g, L.t, b.sc, ns, b.vx_o, b.vy_o, b.vz_o, spec,
-                                                          L.plan_y, twy, b.fft_field);
+        launch_chained(L, k_div_fft_y<2, TS>, grid, 256, smem, g, L.t, b.sc, ns, b.vx_o, b.vy_o, b.vz_o, spec,
+                       L.plan_y, twy, b.fft_field);
       }
       return cudaGetLastError();
     }
@@ -1934,7 +1949,7 @@ static cudaError_t launch_stage_T(const LaunchCtx &L, const SubstepBuffers &b, i
 #define AFID_FFTZ(TXv, INVv)                                                                       \
   do {                                                                                             \
     cudaFuncSetAttribute(k_fft_z<TXv, INVv, TS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-    k_fft_z<TXv, INVv, TS><<<grid, 256, smem, L.stream>>>(g, spec, L.plan_z, twz);                 \
+    launch_chained(L, k_fft_z<TXv, INVv, TS>, grid, 256, smem, g, spec, L.plan_z, twz);                 \
   } while (0)
       if (TXZ == 8) { if (inv) AFID_FFTZ(8, true); else AFID_FFTZ(8, false); }
       else if (TXZ == 4) { if (inv) AFID_FFTZ(4, true); else AFID_FFTZ(4, false); }
@@ -1951,13 +1966,13 @@ static cudaError_t launch_stage_T(const LaunchCtx &L, const SubstepBuffers &b, i
       TS *phi = (TS *)b.phi;
       if (TX == 8) {
         cudaFuncSetAttribute(k_ifft_y<8, TS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        k_ifft_y<8, TS><<<grid, 256, smem, L.stream>>>(g, spec, phi, L.plan_y, twy);
+        launch_chained(L, k_ifft_y<8, TS>, grid, 256, smem, g, spec, phi, L.plan_y, twy);
       } else if (TX == 4) {
         cudaFuncSetAttribute(k_ifft_y<4, TS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        k_ifft_y<4, TS><<<grid, 256, smem, L.stream>>>(g, spec, phi, L.plan_y, twy);
+        launch_chained(L, k_ifft_y<4, TS>, grid, 256, smem, g, spec, phi, L.plan_y, twy);
       } else {
         cudaFuncSetAttribute(k_ifft_y<2, TS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        k_ifft_y<2, TS><<<grid, 256, smem, L.stream>>>(g, spec, phi, L.plan_y, twy);
+        launch_chained(L, k_ifft_y<2, TS>, grid, 256, smem, g, spec, phi, L.plan_y, twy);
       }
       return cudaGetLastError();
     }
@@ -1967,8 +1982,8 @@ static cudaError_t launch_stage_T(const LaunchCtx &L, const SubstepBuffers &b, i
       const int by = 256 / bx;
       dim3 block(bx, by);
       dim3 grid((pairs + bx - 1) / bx, (g.nym + by - 1) / by, g.nzm);
-      k_correct<TS><<<grid, block, 0, L.stream>>>(g, L.t, b.sc, ns, b.vx_o, b.vy_o, b.vz_o, b.vx, b.vy,
-                                                  b.vz, b.pr, (const TS *)b.phi);
+      launch_chained(L, k_correct<TS>, grid, block, 0, g, L.t, b.sc, ns, b.vx_o, b.vy_o, b.vz_o, b.vx, b.vy, b.vz,
+                     b.pr, (const TS *)b.phi);
       return cudaGetLastError();
     }
     case Stage::ExplicitImplicit:
@@ -2012,12 +2027,11 @@ static int reduce_blocks(const Geom &g) {
 
 cudaError_t launch_max_reduce(const LaunchCtx &L, bool div, const double *vx, const double *vy,
                               const double *vz, unsigned long long *out) {
-  cudaMemsetAsync(out, 0, sizeof(unsigned long long), L.stream);
   const int nb = reduce_blocks(L.g);
   if (div)
-    k_max_reduce<true><<<nb, 256, 0, L.stream>>>(L.g, L.t, vx, vy, vz, out);
+    launch_chained(L, k_max_reduce<true>, nb, 256, 0, L.g, L.t, vx, vy, vz, out);
   else
-    k_max_reduce<false><<<nb, 256, 0, L.stream>>>(L.g, L.t, vx, vy, vz, out);
+    launch_chained(L, k_max_reduce<false>, nb, 256, 0, L.g, L.t, vx, vy, vz, out);
   return cudaGetLastError();
 }
 

@@ -62,6 +62,7 @@ __global__ void __launch_bounds__(256)
     k_sal_grad(Geom g, Tables t, const double *__restrict__ vx, const double *__restrict__ vy,
                const double *__restrict__ vz, double *__restrict__ gx, double *__restrict__ gy,
                double *__restrict__ gz) {
+  chain_begin();
   const size_t n = (size_t)g.ldx * g.nym * g.nzm;
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
     const int k = (int)(e % g.ldx);
@@ -88,6 +89,7 @@ __global__ void __launch_bounds__(256)
 __global__ void __launch_bounds__(128)
     k_sal_zint(Geom g, SalGeom sg, SalTables st, const double *__restrict__ gx, const double *__restrict__ gy,
                const double *__restrict__ gz, double *__restrict__ tz) {
+  chain_begin();
   // block per output column (jc, ir): the four source columns and weights are block constants
   const int jc = blockIdx.x % g.nym, ir = blockIdx.x / g.nym;
   const size_t n = (size_t)g.ldx * g.nym * sg.nzmr;
@@ -117,6 +119,7 @@ constexpr int kToRefWarps = 4;
 __global__ void __launch_bounds__(32 * kToRefWarps)
     k_sal_to_ref(Geom g, SalGeom sg, SalTables st, const double *__restrict__ tz, double *__restrict__ vxr,
                  double *__restrict__ gyr, double *__restrict__ gzr) {
+  chain_begin();
   extern __shared__ __align__(16) double sm_to_ref[];
   const int nxm = g.nxm, L = nxm + 4;  // extended rows -2 .. nxm+1 at 0 .. nxm+3
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -190,6 +193,7 @@ __global__ void __launch_bounds__(32 * kToRefWarps)
 __global__ void __launch_bounds__(128)
     k_sal_scan_y(Geom g, SalGeom sg, SalTables st, const double *__restrict__ vy, const double *__restrict__ gyr,
                  double *__restrict__ vyr) {
+  chain_begin();
   const int kr = blockIdx.x * blockDim.x + threadIdx.x, ir = blockIdx.y;
   if (kr >= sg.nxmr) return;
   const int sx = __ldg(st.st[0] + kr), sz = __ldg(st.st[2] + ir);
@@ -224,6 +228,7 @@ __global__ void __launch_bounds__(128)
 __global__ void __launch_bounds__(128)
     k_sal_scan_z(Geom g, SalGeom sg, SalTables st, const double *__restrict__ vz, const double *__restrict__ gzr,
                  double *__restrict__ vzr) {
+  chain_begin();
   const int kr = blockIdx.x * blockDim.x + threadIdx.x, jr = blockIdx.y;
   if (kr >= sg.nxmr) return;
   double v = 0.0;
@@ -265,6 +270,7 @@ __global__ void __launch_bounds__(128)
 // ------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(128)
     k_sal_zc(Geom g, SalGeom sg, SalTables st, const double *__restrict__ sal, double *__restrict__ u) {
+  chain_begin();
   // block per output column (jr, ic): the four refined source columns, their plates and the
   // weights are block constants
   const int jr = blockIdx.x % sg.nymr, ic = blockIdx.x / sg.nymr;
@@ -295,6 +301,7 @@ constexpr int kToCoarseWarps = 4;
 
 __global__ void __launch_bounds__(32 * kToCoarseWarps)
     k_sal_to_coarse(Geom g, SalGeom sg, SalTables st, const double *__restrict__ u, double *__restrict__ salc) {
+  chain_begin();
   // warp per coarse column (j, i), four per block, no block barriers
   extern __shared__ __align__(16) double sm_to_c[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -346,6 +353,7 @@ __global__ void __launch_bounds__(32 * kSalStepWarps)
     k_sal_step(SalGeom sg, SalTables st, const StepCoef *__restrict__ sc_all, int ns, const double *__restrict__ cn_tab,
                const double *__restrict__ sal, const double *__restrict__ vxr, const double *__restrict__ vyr,
                const double *__restrict__ vzr, double *__restrict__ rusal, double *__restrict__ sal_o) {
+  chain_begin();
   constexpr int LD = chunk_ld(MR);
   constexpr int B = MR < 2 ? MR : 2;  // rows per lane whose operands are loaded together
   static_assert(MR % B == 0, "row batches must tile the column");
@@ -447,17 +455,17 @@ __global__ void __launch_bounds__(32 * kSalStepWarps)
 }
 
 template <int MR>
-cudaError_t launch_sal_step_M(const SalCtx &S, cudaStream_t stream, int ns) {
+cudaError_t launch_sal_step_M(const LaunchCtx &L, const SalCtx &S, int ns) {
   const bool two_d = S.sg.nzmr == 1;
   const size_t smem = sal_step_smem(MR, two_d);
   const int ncol = S.sg.nymr * S.sg.nzmr;
   const int nblk = (ncol + kSalStepWarps - 1) / kSalStepWarps;
   if (two_d)
-    k_sal_step<MR, true><<<nblk, 32 * kSalStepWarps, smem, stream>>>(S.sg, S.st, S.sc, ns, S.cn_tab, S.sal, S.vxr,
-                                                                     S.vyr, S.vzr, S.rusal, S.sal_o);
+    launch_chained(L, k_sal_step<MR, true>, nblk, 32 * kSalStepWarps, smem, S.sg, S.st, S.sc, ns, S.cn_tab, S.sal,
+                   S.vxr, S.vyr, S.vzr, S.rusal, S.sal_o);
   else
-    k_sal_step<MR, false><<<nblk, 32 * kSalStepWarps, smem, stream>>>(S.sg, S.st, S.sc, ns, S.cn_tab, S.sal, S.vxr,
-                                                                      S.vyr, S.vzr, S.rusal, S.sal_o);
+    launch_chained(L, k_sal_step<MR, false>, nblk, 32 * kSalStepWarps, smem, S.sg, S.st, S.sc, ns, S.cn_tab, S.sal,
+                   S.vxr, S.vyr, S.vzr, S.rusal, S.sal_o);
   return cudaGetLastError();
 }
 
@@ -470,6 +478,7 @@ cudaError_t launch_sal_step_M(const SalCtx &S, cudaStream_t stream, int ns) {
 __global__ void __launch_bounds__(256)
     k_sal_cfl(SalGeom sg, SalTables st, const double *__restrict__ vxr, const double *__restrict__ vyr,
               const double *__restrict__ vzr, unsigned long long *__restrict__ out) {
+  chain_begin();
   // blocks walk whole refined columns; a thread per row
   const int ncol = sg.nymr * sg.nzmr;
   double m = 0.0;
@@ -492,7 +501,7 @@ __global__ void __launch_bounds__(256)
   __syncthreads();
   if (threadIdx.x == 0) {
     for (int w = 1; w < (int)(blockDim.x >> 5); ++w) m = nan_max(m, wm[w]);
-    atomicMax(out, (unsigned long long)__double_as_longlong(m));
+    reduce_publish(out, m);
   }
 }
 
@@ -571,14 +580,14 @@ int sal_prof_blocks(const SalGeom &sg) {
 
 cudaError_t launch_sal_step(const LaunchCtx &L, const SalCtx &S, int ns) {
   switch (S.sg.MR) {
-    case 1: return launch_sal_step_M<1>(S, L.stream, ns);
-    case 2: return launch_sal_step_M<2>(S, L.stream, ns);
-    case 4: return launch_sal_step_M<4>(S, L.stream, ns);
-    case 8: return launch_sal_step_M<8>(S, L.stream, ns);
-    case 12: return launch_sal_step_M<12>(S, L.stream, ns);
-    case 16: return launch_sal_step_M<16>(S, L.stream, ns);
-    case 24: return launch_sal_step_M<24>(S, L.stream, ns);
-    case 32: return launch_sal_step_M<32>(S, L.stream, ns);
+    case 1: return launch_sal_step_M<1>(L, S, ns);
+    case 2: return launch_sal_step_M<2>(L, S, ns);
+    case 4: return launch_sal_step_M<4>(L, S, ns);
+    case 8: return launch_sal_step_M<8>(L, S, ns);
+    case 12: return launch_sal_step_M<12>(L, S, ns);
+    case 16: return launch_sal_step_M<16>(L, S, ns);
+    case 24: return launch_sal_step_M<24>(L, S, ns);
+    case 32: return launch_sal_step_M<32>(L, S, ns);
   }
   return cudaErrorInvalidValue;
 }
@@ -587,32 +596,30 @@ cudaError_t launch_sal_interp(const LaunchCtx &L, const SalCtx &S, const double 
                               const double *vz) {
   const Geom &g = L.g;
   const size_t nc = (size_t)g.ldx * g.nym * g.nzm;
-  k_sal_grad<<<grid_for(nc, 256), 256, 0, L.stream>>>(g, L.t, vx, vy, vz, S.gx, S.gy, S.gz);
-  k_sal_zint<<<g.nym * S.sg.nzmr, 128, 0, L.stream>>>(g, S.sg, S.st, S.gx, S.gy, S.gz, S.tmp);
+  launch_chained(L, k_sal_grad, grid_for(nc, 256), 256, 0, g, L.t, vx, vy, vz, S.gx, S.gy, S.gz);
+  launch_chained(L, k_sal_zint, g.nym * S.sg.nzmr, 128, 0, g, S.sg, S.st, S.gx, S.gy, S.gz, S.tmp);
   const size_t smem = (size_t)kToRefWarps * 3 * (g.nxm + 4) * sizeof(double);
   if (smem > 48 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(k_sal_to_ref, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
   }
   const int ncr = S.sg.nymr * S.sg.nzmr;
-  k_sal_to_ref<<<(ncr + kToRefWarps - 1) / kToRefWarps, 32 * kToRefWarps, smem, L.stream>>>(g, S.sg, S.st, S.tmp,
-                                                                                            S.vxr, S.gyr, S.gzr);
+  launch_chained(L, k_sal_to_ref, (ncr + kToRefWarps - 1) / kToRefWarps, 32 * kToRefWarps, smem, g, S.sg, S.st, S.tmp,
+                 S.vxr, S.gyr, S.gzr);
   const dim3 gy((S.sg.nxmr + 127) / 128, S.sg.nzmr), gz((S.sg.nxmr + 127) / 128, S.sg.nymr);
-  k_sal_scan_y<<<gy, 128, 0, L.stream>>>(g, S.sg, S.st, vy, S.gyr, S.vyr);
-  k_sal_scan_z<<<gz, 128, 0, L.stream>>>(g, S.sg, S.st, vz, S.gzr, S.vzr);
-  k_sal_zc<<<S.sg.nymr * g.nzm, 128, 0, L.stream>>>(g, S.sg, S.st, S.sal, S.tmp);
+  launch_chained(L, k_sal_scan_y, gy, 128, 0, g, S.sg, S.st, vy, S.gyr, S.vyr);
+  launch_chained(L, k_sal_scan_z, gz, 128, 0, g, S.sg, S.st, vz, S.gzr, S.vzr);
+  launch_chained(L, k_sal_zc, S.sg.nymr * g.nzm, 128, 0, g, S.sg, S.st, S.sal, S.tmp);
   const size_t smc = (size_t)kToCoarseWarps * (S.sg.nxmr + 4) * sizeof(double);
   const int ncc = g.nym * g.nzm;
-  k_sal_to_coarse<<<(ncc + kToCoarseWarps - 1) / kToCoarseWarps, 32 * kToCoarseWarps, smc, L.stream>>>(
-      g, S.sg, S.st, S.tmp, S.salc);
+  launch_chained(L, k_sal_to_coarse, (ncc + kToCoarseWarps - 1) / kToCoarseWarps, 32 * kToCoarseWarps, smc, g, S.sg,
+                 S.st, S.tmp, S.salc);
   return cudaGetLastError();
 }
 
 cudaError_t launch_sal_cfl(const LaunchCtx &L, const SalCtx &S) {
-  cudaError_t e = cudaMemsetAsync(S.red, 0, sizeof(unsigned long long), L.stream);
-  if (e != cudaSuccess) return e;
   const int ncol = S.sg.nymr * S.sg.nzmr;
-  k_sal_cfl<<<ncol < 148 * 8 ? ncol : 148 * 8, 256, 0, L.stream>>>(S.sg, S.st, S.vxr, S.vyr, S.vzr, S.red);
+  launch_chained(L, k_sal_cfl, ncol < 148 * 8 ? ncol : 148 * 8, 256, 0, S.sg, S.st, S.vxr, S.vyr, S.vzr, S.red);
   return cudaGetLastError();
 }
 

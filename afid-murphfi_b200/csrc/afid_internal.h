@@ -32,9 +32,12 @@ struct LaunchCtx {
 // Launch of a kernel whose first statement is chain_begin(): the stream's order is kept by that
 // statement instead of by the launch, so the launch latencies of dependent kernels overlap with the
 // kernels before them.  Small domains are bound by them: a main-loop step of 128 x 64 cells (16
-// kernels) takes 68 us instead of 81, one of 47 x 60 x 50 95 instead of 108.  Not in a captured
+// kernels) takes 62 us instead of 73, one of 47 x 60 x 50 90 instead of 105.  Not in a captured
 // step (L.chained off), where the programmatic edges cost more than plain ones: 25 steps of 24
-// 128 x 64 instances 4.00 ms against 3.87.
+// 128 x 64 instances 4.00 ms against 3.87.  And not above kChainBlocks blocks, where the latency does
+// not count and the order in which waiting blocks are handed to the SMs does: 6 steps with 384^3
+// refined cells took 57 ms chained throughout and 53.7 with this limit or unchained.
+constexpr size_t kChainBlocks = 148 * 32;
 template <typename... P, typename... A>
 inline cudaError_t launch_chained(const LaunchCtx &L, void (*kern)(P...), dim3 grid, dim3 block, size_t smem,
                                   A &&...args) {
@@ -47,7 +50,7 @@ inline cudaError_t launch_chained(const LaunchCtx &L, void (*kern)(P...), dim3 g
   cfg.dynamicSmemBytes = smem;
   cfg.stream = L.stream;
   cfg.attrs = &at;
-  cfg.numAttrs = L.chained ? 1 : 0;
+  cfg.numAttrs = L.chained && (size_t)grid.x * grid.y * grid.z <= kChainBlocks ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
 }
 

@@ -548,6 +548,8 @@ int ctx_create(const afid_grid_t *grid, const afid_params_t *prm, const BatchSpe
   L.div_var = 0;
   L.plan_y = py;
   L.plan_z = pz;
+  L.split_y = fft2_split(nym);
+  L.split_z = fft2_split(bs ? 1 : nzm);
   L.twy = twy;
   L.twz = twz;
   *out = ctx;

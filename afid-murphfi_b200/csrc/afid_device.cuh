@@ -341,10 +341,11 @@ __device__ __forceinline__ typename Cplx<T>::type twiddle(const typename Cplx<T>
   return w;
 }
 
-// One Stockham pass of radix R over N1 registers (input x, output y); NS = product of earlier radices.
+// One Stockham pass of radix R over N1 registers (input x, output y); NS = product of earlier radices,
+// ts = N / N1 for a twiddle table of length N.
 template <bool INV, typename T, int N1, int R, int NS>
 __device__ __forceinline__ void reg_pass(const typename Cplx<T>::type (&x)[N1], typename Cplx<T>::type (&y)[N1],
-                                         const typename Cplx<T>::type *__restrict__ tw) {
+                                         const typename Cplx<T>::type *__restrict__ tw, int ts) {
   using C = typename Cplx<T>::type;
   constexpr int NR = N1 / R;
 #pragma unroll
@@ -356,8 +357,8 @@ __device__ __forceinline__ void reg_pass(const typename Cplx<T>::type (&x)[N1], 
     if constexpr (NS > 1) {
 #pragma unroll
       for (int q = 1; q < R; ++q) {
-        // w_{NS*R}^(q*k) = w_N^(32 * q*k*N1/(NS*R)) for N = 32*N1
-        if (k != 0) a[q] = cmul(a[q], twiddle<INV, T>(tw, 32 * q * k * (N1 / (NS * R))));
+        // w_{NS*R}^(q*k) = w_N^(ts * q*k*N1/(NS*R))
+        if (k != 0) a[q] = cmul(a[q], twiddle<INV, T>(tw, ts * (q * k * (N1 / (NS * R)))));
       }
     }
     dft_small<R, INV, T>(a);
@@ -368,16 +369,16 @@ __device__ __forceinline__ void reg_pass(const typename Cplx<T>::type (&x)[N1], 
 
 template <bool INV, typename T, int N1, int P, int NS>
 __device__ __forceinline__ void reg_fft_rec(typename Cplx<T>::type (&x)[N1],
-                                            const typename Cplx<T>::type *__restrict__ tw) {
+                                            const typename Cplx<T>::type *__restrict__ tw, int ts = 32) {
   using C = typename Cplx<T>::type;
   constexpr RadixList L = radix_list(N1);
   if constexpr (P < L.n) {
     constexpr int R = L.r[P];
     C y[N1];
-    reg_pass<INV, T, N1, R, NS>(x, y, tw);
+    reg_pass<INV, T, N1, R, NS>(x, y, tw, ts);
 #pragma unroll
     for (int q = 0; q < N1; ++q) x[q] = y[q];
-    reg_fft_rec<INV, T, N1, P + 1, NS * R>(x, tw);
+    reg_fft_rec<INV, T, N1, P + 1, NS * R>(x, tw, ts);
   }
 }
 

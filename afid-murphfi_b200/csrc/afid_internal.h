@@ -8,6 +8,13 @@
 
 namespace afid {
 
+// Factors of a transform length for afid_fft2.cu: N = r1 r2 r3 (r3 = 1: two transforms), m = r2 r3;
+// r1 = 0: none that its kernels hold.  Found once a context: the search costs several launches.
+struct FftSplit {
+  int r1, r2, r3, m;
+};
+FftSplit fft2_split(int N);
+
 // Everything a launcher needs that does not change between substeps.
 struct LaunchCtx {
   Geom g;
@@ -25,6 +32,7 @@ struct LaunchCtx {
   int div_var;     // divergence + forward y transform (K2): 0 per-thread loads, 1 tensor copies (FP64
                    // single domain)
   FftPlan plan_y, plan_z;
+  FftSplit split_y, split_z;
   const void *twy, *twz;  // twiddle tables (double2 or float2)
   bool chained = true;    // launch_chained overlaps launches (off while a step is captured)
 };
@@ -107,6 +115,9 @@ bool k1_shape_usable(int M, int v, bool batch, bool two_d);
 enum class Stage { ExplicitImplicit = 0, DivFftY, FftZFwd, Tridiag, FftZInv, IfftY, Correct };
 constexpr int kNumStages = 7;
 cudaError_t launch_stage(const LaunchCtx &L, const SubstepBuffers &b, int ns, Stage st);
+// The transforms of lengths that split into two or three small factors (afid_fft2.cu); false for others.
+template <typename TS>
+bool launch_fft2(const LaunchCtx &L, const SubstepBuffers &b, int ns, Stage st, cudaError_t *err);
 cudaError_t launch_max_reduce(const LaunchCtx &L, bool div, const double *vx, const double *vy,
                               const double *vz, unsigned long long *out);
 cudaError_t launch_globals(const LaunchCtx &L, const double *vx, const double *vy,

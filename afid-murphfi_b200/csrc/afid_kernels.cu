@@ -1918,6 +1918,7 @@ static cudaError_t launch_stage_T(const LaunchCtx &L, const SubstepBuffers &b, i
                      ((st == Stage::FftZFwd || st == Stage::FftZInv) && g.nzm > 1 && !g.batch))) {
     cudaError_t e = cudaSuccess;
     if (launch_warp_fft<TS>(L, b, ns, st, &e)) return e;
+    if (launch_fft2<TS>(L, b, ns, st, &e)) return e;
   }
   switch (st) {
     case Stage::DivFftY: {  // K2 divergence + forward y FFT

@@ -1242,7 +1242,7 @@ cudaError_t launch_k1_cfg(const LaunchCtx &L, const SubstepBuffers &b, int ns, i
   return cudaGetLastError();
 }
 
-// Launch shapes of K1 per M = {1, 2, 4, 8, 12, 16, 24, 32} (rows per lane of the CN solves):
+// Launch shapes of K1 per M = {1, 2, 4, 8, 12, 16, 24, 32, 3, 6} (rows per lane of the CN solves):
 // {threads per column, rows per thread, register cap level, policy (bit 0: the cache hints of
 // tld / nld / sld; bit 1: tables in shared memory; bit 2: adjacent rows per thread; bit 3: the
 // row operands loaded before the staging wait; bit 4: the solves' forward factors loaded before
@@ -1255,10 +1255,12 @@ struct K1Shape {
 };
 constexpr int kK1MaxShapes = 8;
 constexpr int k1_m_index(int M) {
-  return M == 1 ? 0 : M == 2 ? 1 : M == 4 ? 2 : M == 8 ? 3 : M == 12 ? 4 : M == 16 ? 5 : M == 24 ? 6 : 7;
+  return M == 1 ? 0 : M == 2 ? 1 : M == 4 ? 2 : M == 8 ? 3 : M == 12 ? 4 : M == 16 ? 5 : M == 24 ? 6 : M == 32 ? 7
+         : M == 3 ? 8 : 9;
 }
-constexpr int kK1ShapeCount[8] = {1, 5, 8, 8, 8, 8, 6, 5};
-constexpr K1Shape kK1Shapes[8][kK1MaxShapes] = {
+// (the classes of M = 3 and 6, once rows of M = 4 and 8, keep as many entries as those had)
+constexpr int kK1ShapeCount[10] = {1, 5, 8, 8, 8, 8, 6, 5, 8, 8};
+constexpr K1Shape kK1Shapes[10][kK1MaxShapes] = {
     {{32, 1, 0, 0, 1}},                                                                  // M = 1   (nxm <= 32)
     {{64, 1, 0, 0, 1}, {32, 2, 1, 0, 1}, {64, 1, 0, 1, 1}, {64, 1, 0, 1, 2}, {64, 1, 0, 9, 2}},  // M = 2
     {{128, 1, 0, 0, 1}, {64, 2, 1, 0, 1}, {128, 1, 2, 0, 1}, {128, 1, 0, 1, 1},           // M = 4   (<= 128)
@@ -1273,6 +1275,10 @@ constexpr K1Shape kK1Shapes[8][kK1MaxShapes] = {
      {384, 2, 0, 1, 1}, {384, 2, 0, 1, 2}},
     {{256, 4, 1, 0, 1}, {512, 2, 0, 0, 1}, {256, 4, 1, 1, 1}, {512, 2, 0, 1, 1},          // M = 32  (<= 1024)
      {512, 2, 0, 1, 2}},
+    {{128, 1, 0, 0, 1}, {96, 1, 0, 0, 1}, {96, 1, 1, 9, 1}, {128, 1, 1, 25, 1},           // M = 3   (65 .. 96)
+     {96, 1, 1, 9, 2}, {96, 1, 0, 1, 2}, {128, 1, 1, 9, 2}, {96, 1, 2, 1, 1}},
+    {{128, 2, 1, 0, 1}, {128, 2, 1, 25, 1}, {96, 2, 1, 9, 1}, {192, 1, 1, 9, 1},          // M = 6   (129 .. 192)
+     {96, 2, 1, 1, 2}, {192, 1, 1, 9, 2}, {96, 2, 0, 9, 1}, {96, 2, 1, 9, 2}},
 };
 
 template <int M, int V, typename TE, bool TWO_D, bool SAL>
@@ -1313,7 +1319,9 @@ cudaError_t launch_k1_T(const LaunchCtx &L, const SubstepBuffers &b, int ns, int
   switch (L.M) {
     case 1: return launch_k1_M<1, TE, TWO_D, SAL>(L, b, ns, var, ncol);
     case 2: return launch_k1_M<2, TE, TWO_D, SAL>(L, b, ns, var, ncol);
+    case 3: return launch_k1_M<3, TE, TWO_D, SAL>(L, b, ns, var, ncol);
     case 4: return launch_k1_M<4, TE, TWO_D, SAL>(L, b, ns, var, ncol);
+    case 6: return launch_k1_M<6, TE, TWO_D, SAL>(L, b, ns, var, ncol);
     case 8: return launch_k1_M<8, TE, TWO_D, SAL>(L, b, ns, var, ncol);
     case 12: return launch_k1_M<12, TE, TWO_D, SAL>(L, b, ns, var, ncol);
     case 16: return launch_k1_M<16, TE, TWO_D, SAL>(L, b, ns, var, ncol);

@@ -355,7 +355,7 @@ __global__ void __launch_bounds__(32 * kSalStepWarps)
                const double *__restrict__ vzr, double *__restrict__ rusal, double *__restrict__ sal_o) {
   chain_begin();
   constexpr int LD = chunk_ld(MR);
-  constexpr int B = MR < 2 ? MR : 2;  // rows per lane whose operands are loaded together
+  constexpr int B = MR % 2 ? 1 : 2;  // rows per lane whose operands are loaded together
   static_assert(MR % B == 0, "row batches must tile the column");
   extern __shared__ __align__(16) double smem_sal[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -582,7 +582,9 @@ cudaError_t launch_sal_step(const LaunchCtx &L, const SalCtx &S, int ns) {
   switch (S.sg.MR) {
     case 1: return launch_sal_step_M<1>(L, S, ns);
     case 2: return launch_sal_step_M<2>(L, S, ns);
+    case 3: return launch_sal_step_M<3>(L, S, ns);
     case 4: return launch_sal_step_M<4>(L, S, ns);
+    case 6: return launch_sal_step_M<6>(L, S, ns);
     case 8: return launch_sal_step_M<8>(L, S, ns);
     case 12: return launch_sal_step_M<12>(L, S, ns);
     case 16: return launch_sal_step_M<16>(L, S, ns);

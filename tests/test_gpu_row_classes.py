@@ -1,0 +1,56 @@
+"""The wall-normal classes of 96 and 192 rows (three and six rows a lane of the partitioned solves) at
+their edges, against the oracle, and every launch shape of theirs against the first, bit for bit."""
+import numpy as np
+import pytest
+
+import afid_gpu as ag
+from helpers import Case, rel_l2, rel_l2_mod_mean
+from oracle import afid_oracle as o
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("nxm", [64, 65, 95, 96, 97, 128, 129, 160, 191, 192, 193])
+@pytest.mark.parametrize("nym,nzm", [(16, 6), (20, 1)])
+def test_step_at_class_edges(nxm, nym, nzm):
+    case = Case(nxm, nym, nzm, rayt=1e5, dt=1e-3)
+    # the reference's 1 + 1e-15 diagonal leaves phi's mean mode off by rounding times its condition,
+    # which a random start shows in pr above 1e-10 (64 and 128 rows too): the exact solve instead
+    case.g.pin_zero_mode = True
+    s = case.oracle_state(random_velocity=0.1)
+    with case.solver() as gpu:
+        for form in (0, 1):  # both forms of the Poisson solve
+            gpu.upload(s.vx, s.vy, s.vz, s.temp, s.pr)
+            gpu.autotune()
+            gpu.set_k4_form(form)
+            gpu.time_marcher(1e-3, 0)
+            out = gpu.download()
+            if form == 0:
+                first = out
+    o.time_marcher(case.g, s, 1e-3)
+    for f in ("vx", "vy", "vz", "temp"):  # the parity tests' bound
+        assert rel_l2(out[f][..., :nxm], getattr(s, f)[..., :nxm]) < 1e-10, f
+    assert rel_l2_mod_mean(out["pr"][..., :nxm], s.pr[..., :nxm]) < 1e-10
+    for f in ag.Solver.FIELDS:
+        assert np.array_equal(out[f], first[f]), f
+
+
+@pytest.mark.parametrize("shape,precision", [((96, 16, 6), ag.PREC_FP64), ((70, 24, 1), ag.PREC_MIXED),
+                                             ((192, 16, 6), ag.PREC_MIXED), ((150, 16, 8), ag.PREC_FP64)])
+def test_every_shape_bitwise_identical(shape, precision):
+    case = Case(*shape, precision=precision, rayt=1e6, dt=2e-3)
+    s = case.oracle_state(random_velocity=0.1)
+    outs = []
+    with case.solver() as g:
+        info = g.autotune()
+    assert info["ncand"] == 8 and all(us > 0 for *_, us in info["shapes"])
+    for v in range(info["ncand"]):
+        with case.solver() as g:
+            g.set_k1_shape(v)
+            g.upload(s.vx, s.vy, s.vz, s.temp, s.pr)
+            for n in range(2):
+                g.time_marcher(2e-3, n)
+            outs.append(g.download())
+    for got in outs[1:]:
+        for k in ag.Solver.FIELDS:
+            assert np.array_equal(got[k], outs[0][k]), k

@@ -561,9 +561,10 @@ int ctx_run_substep(afid_ctx_t *ctx, int ns) { return run_substep(ctx, ns); }
 int ctx_fail(afid_ctx_t *ctx, cudaError_t e) { return fail_cuda(ctx, e); }
 
 // Time every K1 thread shape on the first `sample` columns and keep the fastest.  The RK3
-// histories point at scratch memory for these launches (K1 updates them in place); the other
-// outputs are intermediates of the next substep or the idle temperature buffer, which the next
-// K1 overwrites, so the state is untouched.  Idle batch slots are timed as active.
+// histories all point at phi for these launches (K1 updates them in place; phi is dead between
+// substeps, as large as one history, and the values do not matter); the other outputs are
+// intermediates of the next substep or the idle temperature buffer, which the next K1 overwrites,
+// so the state is untouched.  Idle batch slots are timed as active.
 int ctx_autotune(afid_ctx_t *ctx, bool force) {
   if (ctx->tuned && !force) return AFID_OK;
   LaunchCtx L = ctx->L;
@@ -572,7 +573,10 @@ int ctx_autotune(afid_ctx_t *ctx, bool force) {
   afid_tune_info_t info{};
   info.ncand = n;
   const int ncol = L.g.nym * L.g.nzm;
-  const int sample = std::min(ncol, 148 * 24);
+  // 18 waves of one-column blocks at four a SM.  With a third of that, shapes of other blocks per SM
+  // were ranked by their last wave (240 x 200 x 180: a two-column shape 38.5 us a sample against
+  // 38.9, 537 us a launch against 487).
+  const int sample = std::min(ncol, 148 * 72);
   info.sample_columns = sample;
   for (int v = 0; v < AFID_TUNE_MAX; ++v) {
     info.threads[v] = v < n ? tpc[v] : 0;
@@ -582,22 +586,14 @@ int ctx_autotune(afid_ctx_t *ctx, bool force) {
     info.us[v] = -1.0;
   }
   if (n > 1) {
-    const size_t tsz = L.mixed ? sizeof(float) : sizeof(double);
-    const size_t per = (size_t)sample * L.g.ldx * tsz;
-    char *scratch = nullptr;
-    AFID_CUDA(ctx, cudaMalloc(&scratch, 4 * per));
     SubstepBuffers b = buffers(ctx);
-    b.rux = scratch;
-    b.ruy = scratch + per;
-    b.ruz = scratch + 2 * per;
-    b.rut = scratch + 3 * per;
+    b.rux = b.ruy = b.ruz = b.rut = ctx->phi;
     L.g.active = nullptr;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
-    cudaError_t e = cudaMemsetAsync(scratch, 0, 4 * per, ctx->stream);
-    if (e == cudaSuccess) e = cudaEventCreate(&e0);
+    cudaError_t e = cudaEventCreate(&e0);
     if (e == cudaSuccess) e = cudaEventCreate(&e1);
     double best = 1e300;
-    constexpr int kReps = 5;
+    constexpr int kReps = 2;
     // two rounds over all candidates, keeping each one's best: the first round also brings the
     // clocks up, which would otherwise bias against the first candidates
     for (int round = 0; round < 2 && e == cudaSuccess; ++round) {
@@ -627,8 +623,6 @@ int ctx_autotune(afid_ctx_t *ctx, bool force) {
       }
     if (e0) cudaEventDestroy(e0);
     if (e1) cudaEventDestroy(e1);
-    cudaError_t ef = cudaFree(scratch);
-    if (e == cudaSuccess) e = ef;
     if (e != cudaSuccess) return fail_cuda(ctx, e);
   }
   ctx->L.k1_var = info.chosen;

@@ -340,8 +340,15 @@ __global__ void __launch_bounds__(32 * kToCoarseWarps)
 // shared memory; the warp then solves the CN system with the factor tables of k_cn_tables
 // (SolveImpEqnUpdate_Sal :408-452) and writes sal_o = sal + increment.  In 2-D the z neighbours
 // are the column itself and those terms vanish; they are left out.
+//
+// Latency-bound: a column's loads wait for DRAM, then its solve is a serial chain, and other
+// resident columns hide both.  Five blocks per SM (at most 102 registers a thread) hide more of it
+// than the compiler's own choice at the price of 12 to 20 spilled bytes in 3-D, none in 2-D: 384^3
+// rows 1013 -> 883 us, 100 x 108 x 160 38.8 -> 34.5 us.  Six blocks spill 56 to 80 bytes from
+// MR = 4 on and measured 978 us; four give 1003 us.
 // ------------------------------------------------------------------------------------------
 constexpr int kSalStepWarps = 4;
+constexpr int kSalStepBlocks = 5;
 
 __host__ __device__ inline size_t sal_step_smem(int MR, bool two_d) {
   (void)two_d;
@@ -349,7 +356,7 @@ __host__ __device__ inline size_t sal_step_smem(int MR, bool two_d) {
 }
 
 template <int MR, bool TWO_D>
-__global__ void __launch_bounds__(32 * kSalStepWarps)
+__global__ void __launch_bounds__(32 * kSalStepWarps, kSalStepBlocks)
     k_sal_step(SalGeom sg, SalTables st, const StepCoef *__restrict__ sc_all, int ns, const double *__restrict__ cn_tab,
                const double *__restrict__ sal, const double *__restrict__ vxr, const double *__restrict__ vyr,
                const double *__restrict__ vzr, double *__restrict__ rusal, double *__restrict__ sal_o) {

@@ -2,10 +2,10 @@
 // CalcMeanProfiles.F90, the spectra of spectra.F90 and the movie planes of MakeMovie*Cut.F90.
 //
 // The fifteen y-z averages written to means.h5 (Tbar, vybar, vzbar, vxT, vyT, vzT, Trms, vxrms,
-// vyrms, vzrms, vxvy, vxvz, vyvz, chiT, epsilon) are reduced in two passes: every block walks
-// through neighbouring x-columns with one thread per wall-normal row k and keeps the fifteen
-// running sums in registers, writes them as one partial row per block, and a second kernel adds the
-// partials in a fixed order (deterministic, no atomics).  The host applies the reference's
+// vyrms, vzrms, vxvy, vxvz, vyvz, chiT, epsilon) are reduced in two passes: every block walks a
+// strided set of x-columns with one thread per wall-normal row k and keeps the fifteen running
+// sums in registers, writes them as one partial row per block, and a second kernel adds the
+// partials in block order (deterministic, no atomics).  The host applies the reference's
 // normalisation (CalcMeanProfiles.F90:88-102, 203-207).
 #include <cuda_runtime.h>
 
@@ -18,141 +18,109 @@ namespace afid {
 
 constexpr int kNumProfiles = 15;
 
-// Sums over columns of the fifteen integrands of CalcMeanProfiles.F90:48-72 (means and second
-// moments), :104-128 (chiT) and :164-199 (epsilon).  A block walks along y through `len` columns of
-// one z index, one thread per row k (blockDim.x >= nxm), and carries what the next column uses
-// again: of the 38 values an integrand set reads, 22 are loaded per column.  With the columns strided
-// over the blocks every value was loaded, and one launch bound of 1024 threads held the fifteen sums
-// and their operands to 64 registers: 252 us at 256 x 192 x 192 cells, now 181.
-// partial[(b*15 + q)*nxm + k].
-template <int MAXT>
-__global__ void __launch_bounds__(MAXT)
+// Sums over the columns [col0, col0 + ncols) of the fifteen integrands of
+// CalcMeanProfiles.F90:48-72 (means and second moments), :104-128 (chiT) and :164-199
+// (epsilon).  Block = one thread per row k (blockDim.x >= nxm); partial[(b*15 + q)*nxm + k].
+__global__ void __launch_bounds__(1024)
     k_mean_partial(Geom g0, Tables t, const double *__restrict__ vx, const double *__restrict__ vy,
-                   const double *__restrict__ vz, const double *__restrict__ temp, int i0, int len, int nseg,
+                   const double *__restrict__ vz, const double *__restrict__ temp, int col0, int ncols,
                    double *__restrict__ partial) {
-  const int nxm = g0.nxm, k = threadIdx.x;
-  if (k >= nxm) return;
-  const int i = i0 + blockIdx.x / nseg, js = blockIdx.x % nseg * len, je = min(js + len, g0.nym);
-  Geom g = g0;
-  bind_instance(g, i);
+  const int k = threadIdx.x;
+  const int nxm = g0.nxm;
   double acc[kNumProfiles];
 #pragma unroll
   for (int q = 0; q < kNumProfiles; ++q) acc[q] = 0.0;
-  const int kp = k + 1, km = max(k - 1, 0), kpc = min(k + 1, nxm - 1);
-  const bool lo = (k == 0), hi = (k == nxm - 1);
-  const double udx3m = __ldg(t.udx3m + k);
-  const double tdx = 0.5 * g.dx / __ldg(t.g3rm + k);                                                     // :113-126
-  const double tdx2 = 0.125 * (g.dx / __ldg(t.g3rm + k)) * (g.dx / __ldg(t.g3rm + k));  // :182-197
-  const double dz = g.dz, dy = g.dy;
-  const int ip = zinc(g, i), im = zdec(g, i);
-  // at (j - 1, i) and (j - 1, i + 1), and at column j: rows k, k + 1, k - 1 of the centre, row k of i +- 1
-  const int jm = wrap_dec(js, g.nym);
-  size_t c = col_off(g, js, i), cip = col_off(g, js, ip), cim = col_off(g, js, im);
-  double txm = vx[col_off(g, jm, i) + k], txm1 = vx[col_off(g, jm, i) + kp];
-  double tm = temp[col_off(g, jm, i) + k], zm = vz[col_off(g, jm, i) + k], zmip = vz[col_off(g, jm, ip) + k];
-  double xc = vx[c + k], xc1 = vx[c + kp], yc = vy[c + k], ycp = vy[c + kpc], ycm = vy[c + km];
-  double yip = vy[cip + k], yim = vy[cim + k], zc = vz[c + k], zip = vz[cip + k], tc = temp[c + k];
-  for (int j = js; j < je; ++j) {
-    const int jp = wrap_inc(j, g.nym);
-    const size_t cjp = col_off(g, jp, i), cjpip = col_off(g, jp, ip), cjpim = col_off(g, jp, im);
-    const double xn = vx[cjp + k], xn1 = vx[cjp + kp], yn = vy[cjp + k], ynp = vy[cjp + kpc], ynm = vy[cjp + km];
-    const double ynip = vy[cjpip + k], ynim = vy[cjpim + k], zn = vz[cjp + k], znip = vz[cjpip + k];
-    const double tn = temp[cjp + k];
-    const double tip = temp[cip + k], tim = temp[cim + k], tcp = temp[c + kpc], tcm = temp[c + km];
-    const double xip = vx[cip + k], xip1 = vx[cip + kp], xim = vx[cim + k], xim1 = vx[cim + kp];
-    const double zcp = vz[c + kpc], zcm = vz[c + km], zipp = vz[cip + kpc], zipm = vz[cip + km];
-    const double vxm = 0.5 * (xc + xc1), vym = 0.5 * (yc + yn), vzm = 0.5 * (zc + zip);
-    acc[0] += tc;
-    acc[1] += vym;
-    acc[2] += vzm;
-    acc[3] += vxm * tc;
-    acc[4] += vym * tc;
-    acc[5] += vzm * tc;
-    acc[6] += tc * tc;
-    acc[7] += 0.5 * (xc * xc + xc1 * xc1);
-    acc[8] += 0.5 * (yc * yc + yn * yn);
-    acc[9] += 0.5 * (zc * zc + zip * zip);
-    acc[10] += 0.25 * (xc + xc1) * (yc + yn);
-    acc[11] += 0.25 * (xc + xc1) * (zc + zip);
-    acc[12] += 0.25 * (yc + yn) * (zc + zip);
-    // chiT: horizontal gradients, then the wall-normal one with the plate values at the walls
-    const double tz = (tip - tim) * 0.5 * dz, ty = (tn - tm) * 0.5 * dy;
-    double tx = tcp - tcm;  // the wall rows repeat their own value
-    if (lo || hi) {
+  if (k < nxm) {
+    const int kp = k + 1, km = k - 1;
+    const bool lo = (k == 0), hi = (k == nxm - 1);
+    const double udx3m = __ldg(t.udx3m + k);
+    const double tdx = 0.5 * g0.dx / __ldg(t.g3rm + k);                       // :113-126
+    const double tdx2 = 0.125 * (g0.dx / __ldg(t.g3rm + k)) * (g0.dx / __ldg(t.g3rm + k));  // :182-197
+    for (int cc = blockIdx.x; cc < ncols; cc += gridDim.x) {
+      const int col = col0 + cc;
+      const int j = col % g0.nym, i = col / g0.nym;
+      Geom g = g0;
+      bind_instance(g, i);
+      const int jp = wrap_inc(j, g.nym), jm = wrap_dec(j, g.nym);
+      const int ip = zinc(g, i), im = zdec(g, i);
+      const size_t c = col_off(g, j, i), cjp = col_off(g, jp, i), cjm = col_off(g, jm, i);
+      const size_t cip = col_off(g, j, ip), cim = col_off(g, j, im);
+      const size_t cjpip = col_off(g, jp, ip), cjpim = col_off(g, jp, im), cjmip = col_off(g, jm, ip);
+      const double tc = temp[c + k];
+      const double vxc = vx[c + k], vxp = vx[c + kp];
+      const double vyc = vy[c + k], vyjp = vy[cjp + k];
+      const double vzc = vz[c + k], vzip = vz[cip + k];
+      const double vxm = 0.5 * (vxc + vxp), vym = 0.5 * (vyc + vyjp), vzm = 0.5 * (vzc + vzip);
+      acc[0] += tc;
+      acc[1] += vym;
+      acc[2] += vzm;
+      acc[3] += vxm * tc;
+      acc[4] += vym * tc;
+      acc[5] += vzm * tc;
+      acc[6] += tc * tc;
+      acc[7] += 0.5 * (vxc * vxc + vxp * vxp);
+      acc[8] += 0.5 * (vyc * vyc + vyjp * vyjp);
+      acc[9] += 0.5 * (vzc * vzc + vzip * vzip);
+      acc[10] += 0.25 * (vxc + vxp) * (vyc + vyjp);
+      acc[11] += 0.25 * (vxc + vxp) * (vzc + vzip);
+      acc[12] += 0.25 * (vyc + vyjp) * (vzc + vzip);
+      // chiT: horizontal gradients, then the wall-normal one with the plate values at the walls
+      const double tz = (temp[cip + k] - temp[cim + k]) * 0.5 * g.dz;
+      const double ty = (temp[cjp + k] - temp[cjm + k]) * 0.5 * g.dy;
+      double tx;
       const size_t pl = (size_t)j + (size_t)g.nym * i;
-      tx += lo ? 2.0 * g.tfixs * (tc - __ldg(t.tempbp + pl)) : 0.0;
-      tx += hi ? 2.0 * g.tfixn * (__ldg(t.temptp + pl) - tc) : 0.0;
+      if (lo)
+        tx = temp[c + 1] - tc + 2.0 * g.tfixs * (tc - __ldg(t.tempbp + pl));
+      else if (hi)
+        tx = tc - temp[c + km] + 2.0 * g.tfixn * (__ldg(t.temptp + pl) - tc);
+      else
+        tx = temp[c + kp] - temp[c + km];
+      acc[13] += tz * tz + ty * ty + (tx * tdx) * (tx * tdx);
+      // epsilon: the seven interior terms, then the wall-normal derivatives of vz and vy
+      const double dz = g.dz, dy = g.dy;
+      const double e1 = (vzip - vzc) * dz;
+      const double a2 = vy[cjpip + k] - vy[cjpim + k], b2 = vy[cip + k] - vy[cim + k];
+      const double a3 = vx[cip + kp] - vx[cim + kp], b3 = vx[cip + k] - vx[cim + k];
+      const double a4 = vz[cjpip + k] - vz[cjmip + k], b4 = vz[cjp + k] - vz[cjm + k];
+      const double e5 = (vyjp - vyc) * dy;
+      const double a6 = vx[cjp + kp] - vx[cjm + kp], b6 = vx[cjp + k] - vx[cjm + k];
+      const double e7 = (vxp - vxc) * udx3m;
+      double eps = e1 * e1 + 0.125 * dz * dz * (a2 * a2 + b2 * b2) + 0.125 * dz * dz * (a3 * a3 + b3 * b3) +
+                   0.125 * dy * dy * (a4 * a4 + b4 * b4) + e5 * e5 + 0.125 * dy * dy * (a6 * a6 + b6 * b6) + e7 * e7;
+      double zxi, zxc, yxj, yxc;  // d/dx of vz at (j, i+1), (j, i) and vy at (j+1, i), (j, i)
+      const double vzip0 = vz[cip + k], vyjp0 = vy[cjp + k];
+      if (lo) {
+        zxi = vz[cip + 1] - vzip0 + g.inslws * 2.0 * (vzip0 - 0.0);
+        zxc = vz[c + 1] - vzc + g.inslws * 2.0 * (vzc - 0.0);
+        yxj = vy[cjp + 1] - vyjp0 + g.inslws * 2.0 * (vyjp0 - g.xminusu);
+        yxc = vy[c + 1] - vyc + g.inslws * 2.0 * (vyc - g.xminusu);
+      } else if (hi) {
+        zxi = vzip0 - vz[cip + km] + g.inslwn * 2.0 * (0.0 - vzip0);
+        zxc = vzc - vz[c + km] + g.inslwn * 2.0 * (0.0 - vzc);
+        yxj = vyjp0 - vy[cjp + km] + g.inslwn * 2.0 * (g.xplusu - vyjp0);
+        yxc = vyc - vy[c + km] + g.inslwn * 2.0 * (g.xplusu - vyc);
+      } else {
+        zxi = vz[cip + kp] - vz[cip + km];
+        zxc = vz[c + kp] - vz[c + km];
+        yxj = vy[cjp + kp] - vy[cjp + km];
+        yxc = vy[c + kp] - vy[c + km];
+      }
+      eps += tdx2 * (zxi * zxi + zxc * zxc) + tdx2 * (yxj * yxj + yxc * yxc);
+      acc[14] += eps;
     }
-    acc[13] += tz * tz + ty * ty + (tx * tdx) * (tx * tdx);
-    // epsilon: the seven interior terms, then the wall-normal derivatives of vz and vy
-    const double e1 = (zip - zc) * dz;
-    const double a2 = ynip - ynim, b2 = yip - yim;
-    const double a3 = xip1 - xim1, b3 = xip - xim;
-    const double a4 = znip - zmip, b4 = zn - zm;
-    const double e5 = (yn - yc) * dy;
-    const double a6 = xn1 - txm1, b6 = xn - txm;
-    const double e7 = (xc1 - xc) * udx3m;
-    double eps = e1 * e1 + 0.125 * dz * dz * (a2 * a2 + b2 * b2) + 0.125 * dz * dz * (a3 * a3 + b3 * b3) +
-                 0.125 * dy * dy * (a4 * a4 + b4 * b4) + e5 * e5 + 0.125 * dy * dy * (a6 * a6 + b6 * b6) + e7 * e7;
-    // d/dx of vz at (j, i+1), (j, i) and vy at (j+1, i), (j, i)
-    double zxi = zipp - zipm, zxc = zcp - zcm, yxj = ynp - ynm, yxc = ycp - ycm;
-    if (lo) {
-      zxi += g.inslws * 2.0 * (zip - 0.0);
-      zxc += g.inslws * 2.0 * (zc - 0.0);
-      yxj += g.inslws * 2.0 * (yn - g.xminusu);
-      yxc += g.inslws * 2.0 * (yc - g.xminusu);
-    }
-    if (hi) {
-      zxi += g.inslwn * 2.0 * (0.0 - zip);
-      zxc += g.inslwn * 2.0 * (0.0 - zc);
-      yxj += g.inslwn * 2.0 * (g.xplusu - yn);
-      yxc += g.inslwn * 2.0 * (g.xplusu - yc);
-    }
-    eps += tdx2 * (zxi * zxi + zxc * zxc) + tdx2 * (yxj * yxj + yxc * yxc);
-    acc[14] += eps;
-    txm = xc;
-    txm1 = xc1;
-    tm = tc;
-    zm = zc;
-    zmip = zip;
-    xc = xn;
-    xc1 = xn1;
-    yc = yn;
-    ycp = ynp;
-    ycm = ynm;
-    yip = ynip;
-    yim = ynim;
-    zc = zn;
-    zip = znip;
-    tc = tn;
-    c = cjp;
-    cip = cjpip;
-    cim = cjpim;
   }
+  if (k < nxm) {
 #pragma unroll
-  for (int q = 0; q < kNumProfiles; ++q) partial[((size_t)blockIdx.x * kNumProfiles + q) * nxm + k] = acc[q];
+    for (int q = 0; q < kNumProfiles; ++q) partial[((size_t)blockIdx.x * kNumProfiles + q) * nxm + k] = acc[q];
+  }
 }
 
-// The partials summed in a fixed order: 32 warps each every 32nd block's, then the 32 sums.  (One thread
-// per profile row over all blocks took 29 us at 592 blocks, eight warps 38 us at 1152.)
-constexpr int kReduceWarps = 32;
-__global__ void __launch_bounds__(32 * kReduceWarps)
-    k_mean_reduce(const double *__restrict__ partial, int nblocks, int nxm, double *__restrict__ out) {
-  __shared__ double part[kReduceWarps][32];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, n = kNumProfiles * nxm;
-  const int e = blockIdx.x * 32 + lane;  // e = q*nxm + k
+__global__ void k_mean_reduce(const double *__restrict__ partial, int nblocks, int nxm, double *__restrict__ out) {
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;  // e = q*nxm + k
+  if (e >= kNumProfiles * nxm) return;
   double s = 0.0;
-  if (e < n) {
-#pragma unroll 4
-    for (int b = warp; b < nblocks; b += kReduceWarps) s += partial[(size_t)b * n + e];
-  }
-  part[warp][lane] = s;
-  __syncthreads();
-  if (warp == 0 && e < n) {
-#pragma unroll
-    for (int w = 1; w < kReduceWarps; ++w) s += part[w][lane];
-    out[e] = s;
-  }
+  for (int b = 0; b < nblocks; ++b) s += partial[(size_t)b * kNumProfiles * nxm + e];
+  out[e] = s;
 }
 
 }  // namespace afid
@@ -166,11 +134,7 @@ namespace afid {
 int ctx_mean_profiles(afid_ctx_t *ctx, int col0, int ncols, double ny_nz, double ren, double pect, double *out) {
   const Geom &g = ctx->L.g;
   const int nxm = g.nxm;
-  // segments of whole z indices' columns: about four blocks of 256 rows an SM, at least four columns
-  const int nz = ncols / g.nym, threads = (nxm + 31) / 32 * 32;
-  const int want = 148 * std::max(1, 1024 / threads);
-  const int parts = std::max(1, std::min(want / nz, (g.nym + 3) / 4));
-  const int len = (g.nym + parts - 1) / parts, nseg = (g.nym + len - 1) / len, nb = nseg * nz;
+  const int nb = std::min(ncols, 148 * 4);
   const size_t need = (size_t)nb * kNumProfiles * nxm + (size_t)kNumProfiles * nxm;
   if (ctx->stats_elems < need) {
     if (ctx->stats_buf) cudaFree(ctx->stats_buf);
@@ -180,10 +144,10 @@ int ctx_mean_profiles(afid_ctx_t *ctx, int col0, int ncols, double ny_nz, double
     ctx->stats_elems = need;
   }
   double *partial = ctx->stats_buf, *sums = ctx->stats_buf + (size_t)nb * kNumProfiles * nxm;
-  auto kern = threads <= 256 ? k_mean_partial<256> : threads <= 512 ? k_mean_partial<512> : k_mean_partial<1024>;
-  kern<<<nb, threads, 0, ctx->stream>>>(g, ctx->L.t, ctx->vx, ctx->vy, ctx->vz, ctx->temp, col0 / g.nym, len, nseg,
-                                        partial);
-  k_mean_reduce<<<(kNumProfiles * nxm + 31) / 32, 32 * kReduceWarps, 0, ctx->stream>>>(partial, nb, nxm, sums);
+  const int threads = (nxm + 31) / 32 * 32;
+  k_mean_partial<<<nb, threads, 0, ctx->stream>>>(g, ctx->L.t, ctx->vx, ctx->vy, ctx->vz, ctx->temp, col0, ncols,
+                                                  partial);
+  k_mean_reduce<<<(kNumProfiles * nxm + 255) / 256, 256, 0, ctx->stream>>>(partial, nb, nxm, sums);
   ctx->launches += 2;
   cudaError_t e = cudaGetLastError();
   std::vector<double> h((size_t)kNumProfiles * nxm);

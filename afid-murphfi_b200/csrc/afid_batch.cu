@@ -31,7 +31,6 @@ struct InstCtl {
 __global__ void __launch_bounds__(256)
     k_batch_cfl(Geom g, Tables t, const double *__restrict__ vx, const double *__restrict__ vy,
                 const double *__restrict__ vz, unsigned long long *__restrict__ out) {
-  chain_begin();
   const int i = blockIdx.y;
   if (!inst_active(g, i)) return;
   bind_instance(g, i);
@@ -78,7 +77,6 @@ __global__ void __launch_bounds__(256)
 __global__ void k_batch_dt(int nslots, unsigned char *__restrict__ active, const InstCtl *__restrict__ ctl,
                            unsigned long long *__restrict__ cfl_bits, const int *__restrict__ ntime,
                            double *__restrict__ dt, double *__restrict__ cfl, int *__restrict__ err) {
-  chain_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nslots || !active[i]) return;
   const unsigned long long bits = cfl_bits[i];
@@ -107,7 +105,6 @@ __global__ void k_batch_dt(int nslots, unsigned char *__restrict__ active, const
 // time += dt (main.F90:313), step counter; a slot that reached its step limit switches off.
 __global__ void k_batch_advance(int nslots, unsigned char *__restrict__ active, const double *__restrict__ dt,
                                 double *__restrict__ time, int *__restrict__ ntime, const int *__restrict__ limit) {
-  chain_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nslots || !active[i]) return;
   time[i] += dt[i];
@@ -282,18 +279,18 @@ int enqueue_step(afid_batch_t *b) {
   if (b->three_d) {
     if (launch_max_reduce(L, false, ctx->vx, ctx->vy, ctx->vz, b->cfl_bits) != cudaSuccess) return AFID_E_CUDA;
   } else {
-    launch_chained(L, k_batch_cfl, dim3(batch_chunks(L.g.nym), b->nslots), 256, 0, L.g, L.t, ctx->vx, ctx->vy,
-                   ctx->vz, b->cfl_bits);
+    k_batch_cfl<<<dim3(batch_chunks(L.g.nym), b->nslots), 256, 0, L.stream>>>(L.g, L.t, ctx->vx, ctx->vy, ctx->vz,
+                                                                              b->cfl_bits);
   }
-  launch_chained(L, k_batch_dt, (b->nslots + 127) / 128, 128, 0, b->nslots, ctx->active_dev, b->ctl, b->cfl_bits,
-                 b->ntime, b->dt, b->cfl, b->err);
+  k_batch_dt<<<(b->nslots + 127) / 128, 128, 0, L.stream>>>(b->nslots, ctx->active_dev, b->ctl, b->cfl_bits, b->ntime,
+                                                            b->dt, b->cfl, b->err);
   ctx->launches += 3;  // with k_batch_advance below
   if (cudaGetLastError() != cudaSuccess) return AFID_E_CUDA;
   int s = ctx_build_cn_batch(ctx, b->dt);
   for (int ns = 0; s == AFID_OK && ns < ctx->nsst; ++ns) s = ctx_run_substep(ctx, ns);
   if (s != AFID_OK) return s;
-  launch_chained(L, k_batch_advance, (b->nslots + 127) / 128, 128, 0, b->nslots, ctx->active_dev, b->dt, b->time,
-                 b->ntime, b->limit);
+  k_batch_advance<<<(b->nslots + 127) / 128, 128, 0, L.stream>>>(b->nslots, ctx->active_dev, b->dt, b->time, b->ntime,
+                                                                 b->limit);
   return cudaGetLastError() == cudaSuccess ? AFID_OK : AFID_E_CUDA;
 }
 
@@ -392,6 +389,7 @@ int afid_batch_create(const afid_input_t *proto, int nslots, int precision, afid
     afid_batch_destroy(b);
     return s;
   }
+  b->ctx->L.chained = false;  // a batch's steps only run captured (launch_chained); the autotuner times the same launches
   cudaError_t e = cudaSuccess;
   auto chk = [&](cudaError_t r) { if (e == cudaSuccess) e = r; };
   if (b->three_d) {
@@ -558,9 +556,7 @@ int afid_batch_step(afid_batch_t *b, int nsteps) {
       cudaGraph_t graph = nullptr;
       cudaError_t e = cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal);
       if (e != cudaSuccess) return ctx_fail(ctx, e);
-      ctx->L.chained = false;  // see launch_chained
       int s = enqueue_step(b);
-      ctx->L.chained = true;
       e = cudaStreamEndCapture(ctx->stream, &graph);
       ctx->temp = temp0;
       ctx->temp_o = tempo0;

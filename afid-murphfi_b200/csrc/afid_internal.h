@@ -34,7 +34,7 @@ struct LaunchCtx {
   FftPlan plan_y, plan_z;
   FftSplit split_y, split_z;
   const void *twy, *twz;  // twiddle tables (double2 or float2)
-  bool chained = true;    // launch_chained overlaps launches (off while a step is captured)
+  bool chained = true;    // launch_chained overlaps launches (off in a batch, whose steps are captured)
 };
 
 // Launch of a kernel whose first statement is chain_begin(): the stream's order is kept by that

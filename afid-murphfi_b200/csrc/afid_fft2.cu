@@ -139,7 +139,7 @@ __device__ __forceinline__ int last(const typename Cplx<T>::type *s, typename Cp
 template <int RMAX, bool THREE, bool INV, typename TS>
 __global__ void __launch_bounds__(block_threads(128 / (2 * (int)sizeof(TS)), RMAX, THREE),
                                   blocks_per_sm<TS>(128 / (2 * (int)sizeof(TS)), RMAX, THREE))
-    k_fft2_z(Geom g, typename Cplx<TS>::type *__restrict__ spec, Split f,
+    k_fft2_z(Geom g, typename Cplx<TS>::type *spec, Split f,
              const typename Cplx<TS>::type *__restrict__ tw) {
   chain_begin();
   using C = typename Cplx<TS>::type;
@@ -182,9 +182,9 @@ __global__ void __launch_bounds__(block_threads(128 / (2 * (int)sizeof(TS)), RMA
 // points (8 packed pairs) at one z index.
 template <int RMAX, typename TS>
 __global__ void __launch_bounds__(block_threads(8, RMAX, false), blocks_per_sm<TS>(8, RMAX, false))
-    k_fft2_div(Geom g0, Tables t, const StepCoef *__restrict__ sc_all, int ns, const double *__restrict__ vx,
-               const double *__restrict__ vy, const double *__restrict__ vz, typename Cplx<TS>::type *__restrict__ spec, Split f,
-               const typename Cplx<TS>::type *__restrict__ tw, const double *__restrict__ field) {
+    k_fft2_div(Geom g0, Tables t, const StepCoef *sc_all, int ns, const double *vx,
+               const double *vy, const double *vz, typename Cplx<TS>::type *spec, Split f,
+               const typename Cplx<TS>::type *__restrict__ tw, const double *field) {
   chain_begin();
   using C = typename Cplx<TS>::type;
   constexpr int W = 8;
@@ -213,7 +213,7 @@ __global__ void __launch_bounds__(block_threads(8, RMAX, false), blocks_per_sm<T
       for (int j = row0; j < N; j += dj) put(j, 0.0, 0.0);
     } else if (field) {  // spectra: the field itself
       for (int j = row0; j < N; j += dj) {
-        const double2 v = __ldg(reinterpret_cast<const double2 *>(field + c0 + (size_t)j * g.ldx));
+        const double2 v = *reinterpret_cast<const double2 *>(field + c0 + (size_t)j * g.ldx);
         put(j, v.x, (kk + 1 < nxm) ? v.y : 0.0);
       }
     } else {
@@ -222,12 +222,12 @@ __global__ void __launch_bounds__(block_threads(8, RMAX, false), blocks_per_sm<T
 #pragma unroll 4
       for (int j = row0; j < N; j += dj) {
         const size_t o = (size_t)j * g.ldx, op = (size_t)wrap_inc(j, N) * g.ldx;
-        const double2 zi = __ldg(reinterpret_cast<const double2 *>(vz + ci + o));
-        const double2 zc = __ldg(reinterpret_cast<const double2 *>(vz + c0 + o));
-        const double2 yj = __ldg(reinterpret_cast<const double2 *>(vy + c0 + op));
-        const double2 yc = __ldg(reinterpret_cast<const double2 *>(vy + c0 + o));
-        const double2 xc = __ldg(reinterpret_cast<const double2 *>(vx + c0 + o));
-        const double x2 = __ldg(vx + c0 + o + d2);
+        const double2 zi = *reinterpret_cast<const double2 *>(vz + ci + o);
+        const double2 zc = *reinterpret_cast<const double2 *>(vz + c0 + o);
+        const double2 yj = *reinterpret_cast<const double2 *>(vy + c0 + op);
+        const double2 yc = *reinterpret_cast<const double2 *>(vy + c0 + o);
+        const double2 xc = *reinterpret_cast<const double2 *>(vx + c0 + o);
+        const double x2 = vx[c0 + o + d2];
         const double dv1 = ((zi.y - zc.y) * g.dz + (yj.y - yc.y) * g.dy + (x2 - xc.y) * ux.y) * usdtal;
         put(j, ((zi.x - zc.x) * g.dz + (yj.x - yc.x) * g.dy + (xc.y - xc.x) * ux.x) * usdtal, two ? dv1 : 0.0);
       }
@@ -277,7 +277,7 @@ __global__ void __launch_bounds__(block_threads(8, RMAX, false), blocks_per_sm<T
 // in shared memory would have to be kept until every row's first transform is done).
 template <int RMAX, bool THREE, typename TS>
 __global__ void __launch_bounds__(block_threads(8, RMAX, THREE), blocks_per_sm<TS>(8, RMAX, THREE))
-    k_fft2_ify(Geom g, const typename Cplx<TS>::type *__restrict__ spec, TS *__restrict__ phi, Split f,
+    k_fft2_ify(Geom g, const typename Cplx<TS>::type *spec, TS *phi, Split f,
                const typename Cplx<TS>::type *__restrict__ tw) {
   chain_begin();
   using C = typename Cplx<TS>::type;

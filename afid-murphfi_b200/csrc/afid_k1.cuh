@@ -10,11 +10,11 @@
 
 namespace afid {
 
-// Loads by cache policy.  H = 0: read-only data through the non-coherent path (__ldg) and the
-// RK3 histories by plain loads.  H = 1: the tables every block reads (metric coefficients, CN
-// factors) are kept in L1 with the evict_last priority, and the data each block reads once (RK3
+// Loads by cache policy.  H = 0: no hints.  H = 1: the tables every block reads (metric coefficients,
+// CN factors) are kept in L1 with the evict_last priority, and the data each block reads once (RK3
 // histories, single-row neighbours) bypasses L1 (no_allocate), so the streaming data does not
-// evict the tables.  H = 2 (tld only): the tables sit in shared memory; plain loads.
+// evict the tables.  H = 2: the tables sit in shared memory; plain loads.
+// tld: metric coefficients, which nothing writes after the context's creation: the read-only path.
 template <int H> __device__ __forceinline__ double tld(const double *p) {
   if constexpr (H == 2) {  // tables staged in shared memory (k_explicit_implicit_p)
     return *p;
@@ -26,13 +26,24 @@ template <int H> __device__ __forceinline__ double tld(const double *p) {
     return __ldg(p);
   }
 }
+// cld: CN factors, written by k_cn_tables; nld: fields, written by the projection.  K1 may be resident
+// while either runs (chain_begin), so both are coherent loads that stay behind it.
+template <int H> __device__ __forceinline__ double cld(const double *p) {
+  if constexpr (H == 1) {
+    double v;
+    asm volatile("ld.global.L1::evict_last.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
+    return v;
+  } else {
+    return *p;
+  }
+}
 template <int H> __device__ __forceinline__ double nld(const double *p) {
   if constexpr (H != 0) {
     double v;
-    asm("ld.global.nc.L1::no_allocate.f64 %0, [%1];" : "=d"(v) : "l"(p));
+    asm volatile("ld.global.L1::no_allocate.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
     return v;
   } else {
-    return __ldg(p);
+    return *p;
   }
 }
 // Read-write streaming data (the histories, rewritten later by the same thread): coherent loads.
@@ -66,8 +77,8 @@ struct CnFwd {
   __device__ __forceinline__ void load(const double *__restrict__ T, int lane) {
 #pragma unroll
     for (int q = 1; q < M; ++q) {
-      inv[q] = tld<H>(T + 64 * M + q * 32 + lane);
-      if (q >= 2) a[q] = tld<H>(T + 32 * M + q * 32 + lane);
+      inv[q] = cld<H>(T + 64 * M + q * 32 + lane);
+      if (q >= 2) a[q] = cld<H>(T + 32 * M + q * 32 + lane);
     }
   }
 };
@@ -84,38 +95,38 @@ __device__ __forceinline__ void cn_solve_chunk(double *__restrict__ s, const dou
 #pragma unroll
   for (int q = 0; q < M; ++q) y[q] = s[q * LD + lane];
   if constexpr (M > 1) {
-    y[1] = y[1] * (PRE ? fw->inv[1] : tld<H>(Tinv + 32 + lane));
+    y[1] = y[1] * (PRE ? fw->inv[1] : cld<H>(Tinv + 32 + lane));
 #pragma unroll
     for (int q = 2; q < M; ++q)
-      y[q] = (y[q] - (PRE ? fw->a[q] : tld<H>(Ta + q * 32 + lane)) * y[q - 1]) *
-             (PRE ? fw->inv[q] : tld<H>(Tinv + q * 32 + lane));
+      y[q] = (y[q] - (PRE ? fw->a[q] : cld<H>(Ta + q * 32 + lane)) * y[q - 1]) *
+             (PRE ? fw->inv[q] : cld<H>(Tinv + q * 32 + lane));
 #pragma unroll
-    for (int q = M - 2; q >= 1; --q) y[q] = y[q] - tld<H>(Tcp + q * 32 + lane) * y[q + 1];
+    for (int q = M - 2; q >= 1; --q) y[q] = y[q] - cld<H>(Tcp + q * 32 + lane) * y[q + 1];
   }
   double D;
   if constexpr (M > 1) {
     double yprev = __shfl_up_sync(0xffffffffu, y[M - 1], 1);
     if (lane == 0) yprev = 0.0;
-    D = y[0] - tld<H>(Tl + lane) * yprev - tld<H>(Tl + 32 + lane) * y[1];
+    D = y[0] - cld<H>(Tl + lane) * yprev - cld<H>(Tl + 32 + lane) * y[1];
   } else {
     D = y[0];
   }
-  double delta = D * tld<H>(Tl + 64 + lane);
+  double delta = D * cld<H>(Tl + 64 + lane);
 #pragma unroll
   for (int lev = 0, h = 1; lev < 5; ++lev, h <<= 1) {
     double dm = __shfl_up_sync(0xffffffffu, delta, h);
     double dp = __shfl_down_sync(0xffffffffu, delta, h);
     if (lane < h) dm = 0.0;
     if (lane + h >= 32) dp = 0.0;
-    delta = (delta - tld<H>(Tl + 96 + lev * 32 + lane) * dm - tld<H>(Tl + 256 + lev * 32 + lane) * dp) *
-            tld<H>(Tl + 416 + lev * 32 + lane);
+    delta = (delta - cld<H>(Tl + 96 + lev * 32 + lane) * dm - cld<H>(Tl + 256 + lev * 32 + lane) * dp) *
+            cld<H>(Tl + 416 + lev * 32 + lane);
   }
   double xnext = __shfl_down_sync(0xffffffffu, delta, 1);
   if (lane == 31) xnext = 0.0;
   s[lane] = delta;
 #pragma unroll
   for (int q = 1; q < M; ++q)
-    s[q * LD + lane] = y[q] + tld<H>(Tv + q * 32 + lane) * delta + tld<H>(Tw + q * 32 + lane) * xnext;
+    s[q * LD + lane] = y[q] + cld<H>(Tv + q * 32 + lane) * delta + cld<H>(Tw + q * 32 + lane) * xnext;
 }
 
 // Two columns with the same matrix (s0, s1: chunk layout as above) solved by one warp: every
@@ -133,18 +144,18 @@ __device__ __forceinline__ void cn_solve_chunk2(double *__restrict__ s0, double 
     z[q] = s1[q * LD + lane];
   }
   if constexpr (M > 1) {
-    const double i1 = tld<H>(Tinv + 32 + lane);
+    const double i1 = cld<H>(Tinv + 32 + lane);
     y[1] = y[1] * i1;
     z[1] = z[1] * i1;
 #pragma unroll
     for (int q = 2; q < M; ++q) {
-      const double a = tld<H>(Ta + q * 32 + lane), iv = tld<H>(Tinv + q * 32 + lane);
+      const double a = cld<H>(Ta + q * 32 + lane), iv = cld<H>(Tinv + q * 32 + lane);
       y[q] = (y[q] - a * y[q - 1]) * iv;
       z[q] = (z[q] - a * z[q - 1]) * iv;
     }
 #pragma unroll
     for (int q = M - 2; q >= 1; --q) {
-      const double cp = tld<H>(Tcp + q * 32 + lane);
+      const double cp = cld<H>(Tcp + q * 32 + lane);
       y[q] = y[q] - cp * y[q + 1];
       z[q] = z[q] - cp * z[q + 1];
     }
@@ -154,14 +165,14 @@ __device__ __forceinline__ void cn_solve_chunk2(double *__restrict__ s0, double 
     double yprev = __shfl_up_sync(0xffffffffu, y[M - 1], 1);
     double zprev = __shfl_up_sync(0xffffffffu, z[M - 1], 1);
     if (lane == 0) yprev = zprev = 0.0;
-    const double l0 = tld<H>(Tl + lane), l1 = tld<H>(Tl + 32 + lane);
+    const double l0 = cld<H>(Tl + lane), l1 = cld<H>(Tl + 32 + lane);
     Dy = y[0] - l0 * yprev - l1 * y[1];
     Dz = z[0] - l0 * zprev - l1 * z[1];
   } else {
     Dy = y[0];
     Dz = z[0];
   }
-  const double l2 = tld<H>(Tl + 64 + lane);
+  const double l2 = cld<H>(Tl + 64 + lane);
   double dy = Dy * l2, dz = Dz * l2;
 #pragma unroll
   for (int lev = 0, h = 1; lev < 5; ++lev, h <<= 1) {
@@ -169,8 +180,8 @@ __device__ __forceinline__ void cn_solve_chunk2(double *__restrict__ s0, double 
     double zm = __shfl_up_sync(0xffffffffu, dz, h), zp = __shfl_down_sync(0xffffffffu, dz, h);
     if (lane < h) ym = zm = 0.0;
     if (lane + h >= 32) yp = zp = 0.0;
-    const double lm = tld<H>(Tl + 96 + lev * 32 + lane), lp = tld<H>(Tl + 256 + lev * 32 + lane),
-                 li = tld<H>(Tl + 416 + lev * 32 + lane);
+    const double lm = cld<H>(Tl + 96 + lev * 32 + lane), lp = cld<H>(Tl + 256 + lev * 32 + lane),
+                 li = cld<H>(Tl + 416 + lev * 32 + lane);
     dy = (dy - lm * ym - lp * yp) * li;
     dz = (dz - lm * zm - lp * zp) * li;
   }
@@ -180,7 +191,7 @@ __device__ __forceinline__ void cn_solve_chunk2(double *__restrict__ s0, double 
   s1[lane] = dz;
 #pragma unroll
   for (int q = 1; q < M; ++q) {
-    const double v = tld<H>(Tv + q * 32 + lane), w = tld<H>(Tw + q * 32 + lane);
+    const double v = cld<H>(Tv + q * 32 + lane), w = cld<H>(Tw + q * 32 + lane);
     s0[q * LD + lane] = y[q] + v * dy + w * ynext;
     s1[q * LD + lane] = z[q] + v * dz + w * znext;
   }
@@ -444,13 +455,13 @@ constexpr int k1_min_blocks() {
 }
 template <int M, int TPC, int RPT, typename TE, bool TWO_D, int CAP, bool SAL, int POL>
 __global__ void __launch_bounds__(TPC, k1_min_blocks<CAP, TPC>())
-    k_explicit_implicit(Geom g0, Tables t, const StepCoef *__restrict__ sc_all, int ns,
-                        const double *__restrict__ cn_tab, const double *__restrict__ vx,
-                        const double *__restrict__ vy, const double *__restrict__ vz,
-                        const double *__restrict__ temp, const double *__restrict__ pr,
-                        TE *__restrict__ rux, TE *__restrict__ ruy, TE *__restrict__ ruz,
-                        TE *__restrict__ rut, double *__restrict__ vx_o, double *__restrict__ vy_o,
-                        double *__restrict__ vz_o, double *__restrict__ temp_o, int *__restrict__ err) {
+    k_explicit_implicit(Geom g0, Tables t, const StepCoef *sc_all, int ns,
+                        const double *cn_tab, const double *vx,
+                        const double *vy, const double *vz,
+                        const double *temp, const double *pr,
+                        TE *rux, TE *ruy, TE *ruz,
+                        TE *rut, double *vx_o, double *vy_o,
+                        double *vz_o, double *temp_o, int *err) {
   chain_begin();
   constexpr int LD = chunk_ld(M);
   constexpr int FLD = LD * M;
@@ -550,9 +561,9 @@ __global__ void __launch_bounds__(TPC, k1_min_blocks<CAP, TPC>())
     const int k = ADJ ? RPT * tc : tc;
     if (k < g.nxm) {
       rte = row_tab<H>(t, k);
-      rse[0] = (k >= 1) ? tld<H>(TX + k - 1) : 0.0;
-      rse[1] = tld<H>(TY + k);
-      rse[2] = tld<H>(TT + k);
+      rse[0] = (k >= 1) ? cld<H>(TX + k - 1) : 0.0;
+      rse[1] = cld<H>(TY + k);
+      rse[2] = cld<H>(TT + k);
     }
   }
 
@@ -592,9 +603,9 @@ __global__ void __launch_bounds__(TPC, k1_min_blocks<CAP, TPC>())
       double sb = 0.0;
       if constexpr (SAL) sb = sbv[p];
       // all four right-hand sides from the staged columns before anything is stored
-      const double sx = (EARLY && p == 0) ? rse[0] : ((k >= 1) ? tld<H>(TX + k - 1) : 0.0);
-      const double sy = (EARLY && p == 0) ? rse[1] : tld<H>(TY + k);
-      const double st = (EARLY && p == 0) ? rse[2] : tld<H>(TT + k);
+      const double sx = (EARLY && p == 0) ? rse[0] : ((k >= 1) ? cld<H>(TX + k - 1) : 0.0);
+      const double sy = (EARLY && p == 0) ? rse[1] : cld<H>(TY + k);
+      const double st = (EARLY && p == 0) ? rse[2] : cld<H>(TT + k);
       rr[p][0] = (k >= 1) ? rhs_vx<TE, TWO_D, SAL, H>(g, rt, sc, k, X, Y, Z, T, P, u0, q0, sb) * sx : 0.0;
       rr[p][1] = rhs_vy<TE, TWO_D, SAL, H>(g, rt, sc, k, X, Y, Z, T, P, zd, vv[p][2], u1, q1, sb) * sy;
       rr[p][2] = rhs_vz<TE, TWO_D, SAL, H>(g, rt, sc, k, X, Y, Z, T, P, yd, pim, u2, q2, sb) * sy;
@@ -689,13 +700,13 @@ __host__ __device__ inline size_t k1y2_smem(int M, bool two_d) {
 
 template <int M, int TPC, int RPT, typename TE, bool TWO_D, int CAP, bool SAL, int POL>
 __global__ void __launch_bounds__(TPC, k1_min_blocks<CAP, TPC>())
-    k_explicit_implicit_y2(Geom g0, Tables t, const StepCoef *__restrict__ sc_all, int ns,
-                           const double *__restrict__ cn_tab, const double *__restrict__ vx,
-                           const double *__restrict__ vy, const double *__restrict__ vz,
-                           const double *__restrict__ temp, const double *__restrict__ pr,
-                           TE *__restrict__ rux, TE *__restrict__ ruy, TE *__restrict__ ruz,
-                           TE *__restrict__ rut, double *__restrict__ vx_o, double *__restrict__ vy_o,
-                           double *__restrict__ vz_o, double *__restrict__ temp_o, int *__restrict__ err) {
+    k_explicit_implicit_y2(Geom g0, Tables t, const StepCoef *sc_all, int ns,
+                           const double *cn_tab, const double *vx,
+                           const double *vy, const double *vz,
+                           const double *temp, const double *pr,
+                           TE *rux, TE *ruy, TE *ruz,
+                           TE *rut, double *vx_o, double *vy_o,
+                           double *vz_o, double *temp_o, int *err) {
   chain_begin();
   constexpr int LD = chunk_ld(M);
   constexpr int FLD = LD * M;
@@ -794,9 +805,9 @@ __global__ void __launch_bounds__(TPC, k1_min_blocks<CAP, TPC>())
   if constexpr (EARLY) {
     if (tc < g.nxm) {
       rte = row_tab<H>(t, tc);
-      rse[0] = (tc >= 1) ? tld<H>(TX + tc - 1) : 0.0;
-      rse[1] = tld<H>(TY + tc);
-      rse[2] = tld<H>(TT + tc);
+      rse[0] = (tc >= 1) ? cld<H>(TX + tc - 1) : 0.0;
+      rse[1] = cld<H>(TY + tc);
+      rse[2] = cld<H>(TT + tc);
     }
   }
   bool ok = mbar_wait(&bar, 0, kSpinLimit);
@@ -844,9 +855,9 @@ __global__ void __launch_bounds__(TPC, k1_min_blocks<CAP, TPC>())
         pjm = c == 0 ? sv[p][0] : C(PRC)[k];
         double sb = 0.0;
         if constexpr (SAL) sb = sbv[p][c];
-        const double sx = (EARLY && p == 0) ? rse[0] : ((k >= 1) ? tld<H>(TX + k - 1) : 0.0);
-        const double sy = (EARLY && p == 0) ? rse[1] : tld<H>(TY + k);
-        const double st = (EARLY && p == 0) ? rse[2] : tld<H>(TT + k);
+        const double sx = (EARLY && p == 0) ? rse[0] : ((k >= 1) ? cld<H>(TX + k - 1) : 0.0);
+        const double sy = (EARLY && p == 0) ? rse[1] : cld<H>(TY + k);
+        const double st = (EARLY && p == 0) ? rse[2] : cld<H>(TT + k);
         rr[p][c][0] =
             (k >= 1) ? rhs_vx<TE, TWO_D, SAL, H>(g, rt, sc, k, X, Y, Z, T, P, uu[p][c][0], q0, sb) * sx : 0.0;
         rr[p][c][1] = rhs_vy<TE, TWO_D, SAL, H>(g, rt, sc, k, X, Y, Z, T, P, zd, pjm, uu[p][c][1], q1, sb) * sy;
@@ -992,13 +1003,13 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
 
 template <int M, int TPC, int RPT, typename TE, bool TWO_D, bool SAL, int G>
 __global__ void __launch_bounds__(TPC * G, 1)
-    k_explicit_implicit_p(Geom g0, Tables t, const StepCoef *__restrict__ sc_all, int ns,
-                          const double *__restrict__ cn_tab, const double *__restrict__ vx,
-                          const double *__restrict__ vy, const double *__restrict__ vz,
-                          const double *__restrict__ temp, const double *__restrict__ pr,
-                          TE *__restrict__ rux, TE *__restrict__ ruy, TE *__restrict__ ruz,
-                          TE *__restrict__ rut, double *__restrict__ vx_o, double *__restrict__ vy_o,
-                          double *__restrict__ vz_o, double *__restrict__ temp_o, int *__restrict__ err,
+    k_explicit_implicit_p(Geom g0, Tables t, const StepCoef *sc_all, int ns,
+                          const double *cn_tab, const double *vx,
+                          const double *vy, const double *vz,
+                          const double *temp, const double *pr,
+                          TE *rux, TE *ruy, TE *ruz,
+                          TE *rut, double *vx_o, double *vy_o,
+                          double *vz_o, double *temp_o, int *err,
                           int ncol) {
   chain_begin();
   constexpr int LD = chunk_ld(M);

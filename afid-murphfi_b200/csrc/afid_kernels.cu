@@ -63,8 +63,8 @@ struct CnBuildArgs {
   const unsigned char *active;
 };
 
-__global__ void k_cn_tables(CnBuildArgs args, int M, double *__restrict__ tab,
-                            StepCoef *__restrict__ sc) {
+__global__ void k_cn_tables(CnBuildArgs args, int M, double *tab,
+                            StepCoef *sc) {
   chain_begin();
   const int lane = threadIdx.x;
   const int m = blockIdx.x % args.nmat;
@@ -178,10 +178,10 @@ __global__ void k_cn_tables(CnBuildArgs args, int M, double *__restrict__ tab,
 // ------------------------------------------------------------------------------------------
 template <int TX, typename TS>
 __global__ void __launch_bounds__(256)
-    k_div_fft_y(Geom g0, Tables t, const StepCoef *__restrict__ sc_all, int ns,
-                const double *__restrict__ vx, const double *__restrict__ vy,
-                const double *__restrict__ vz, typename Cplx<TS>::type *__restrict__ spec,
-                FftPlan pl, const typename Cplx<TS>::type *__restrict__ tw, const double *__restrict__ field) {
+    k_div_fft_y(Geom g0, Tables t, const StepCoef *sc_all, int ns,
+                const double *vx, const double *vy,
+                const double *vz, typename Cplx<TS>::type *spec,
+                FftPlan pl, const typename Cplx<TS>::type *__restrict__ tw, const double *field) {
   chain_begin();
   using C = typename Cplx<TS>::type;
   extern __shared__ __align__(16) unsigned char smem_raw_k2[];
@@ -201,13 +201,13 @@ __global__ void __launch_bounds__(256)
   for (int j = threadIdx.x / TX; j < N; j += blockDim.x / TX) {
     double dv = 0.0;
     if (k < g.nxm && field) {
-      dv = __ldg(field + col_off(g, j, i) + k);
+      dv = field[col_off(g, j, i) + k];
     } else if (k < g.nxm) {
       const int jp = wrap_inc(j, N);
       const size_t c = col_off(g, j, i), cjp = col_off(g, jp, i), cip = col_off(g, j, ip);
-      const double dqcap = (__ldg(vz + cip + k) - __ldg(vz + c + k)) * g.dz +
-                           (__ldg(vy + cjp + k) - __ldg(vy + c + k)) * g.dy +
-                           (__ldg(vx + c + k + 1) - __ldg(vx + c + k)) * __ldg(t.udx3m + k);
+      const double dqcap = (vz[cip + k] - vz[c + k]) * g.dz +
+                           (vy[cjp + k] - vy[c + k]) * g.dy +
+                           (vx[c + k + 1] - vx[c + k]) * __ldg(t.udx3m + k);
       dv = dqcap * usdtal;
     }
     TS *d = reinterpret_cast<TS *>(&b0[(size_t)(tx >> 1) * N + j]);
@@ -241,7 +241,7 @@ __global__ void __launch_bounds__(256)
 // K3 / K5: z c2c FFT in place on the spectrum.  Block = (x tile of TXZ points, ky).
 template <int TXZ, bool INV, typename TS>
 __global__ void __launch_bounds__(256)
-    k_fft_z(Geom g, typename Cplx<TS>::type *__restrict__ spec, FftPlan pl,
+    k_fft_z(Geom g, typename Cplx<TS>::type *spec, FftPlan pl,
             const typename Cplx<TS>::type *__restrict__ tw) {
   chain_begin();
   using C = typename Cplx<TS>::type;
@@ -281,8 +281,8 @@ __global__ void __launch_bounds__(256)
 // ------------------------------------------------------------------------------------------
 template <int M, int WPB, typename TS>
 __global__ void __launch_bounds__(WPB * 32)
-    k_tridiag_pressure(Geom g, Tables t, typename Cplx<TS>::type *__restrict__ spec,
-                       int *__restrict__ err) {
+    k_tridiag_pressure(Geom g, Tables t, typename Cplx<TS>::type *spec,
+                       int *err) {
   chain_begin();
   using C = typename Cplx<TS>::type;
   extern __shared__ double smem_k4[];
@@ -432,7 +432,7 @@ __global__ void __launch_bounds__(WPB * 32)
 // Re -> phi(k0), Im -> phi(k0+1).
 template <int TX, typename TS>
 __global__ void __launch_bounds__(256)
-    k_ifft_y(Geom g, const typename Cplx<TS>::type *__restrict__ spec, TS *__restrict__ phi,
+    k_ifft_y(Geom g, const typename Cplx<TS>::type *spec, TS *phi,
              FftPlan pl, const typename Cplx<TS>::type *__restrict__ tw) {
   chain_begin();
   using C = typename Cplx<TS>::type;
@@ -492,10 +492,10 @@ struct Vec2<float> {
 // vector loads and stores; the x-neighbours of the pair come from the adjacent threads.
 template <typename TS>
 __global__ void __launch_bounds__(256)
-    k_correct(Geom g0, Tables t, const StepCoef *__restrict__ sc_all, int ns,
-              const double *__restrict__ vxh, const double *__restrict__ vyh,
-              const double *__restrict__ vzh, double *__restrict__ vx, double *__restrict__ vy,
-              double *__restrict__ vz, double *__restrict__ pr, const TS *__restrict__ phi) {
+    k_correct(Geom g0, Tables t, const StepCoef *sc_all, int ns,
+              const double *vxh, const double *vyh,
+              const double *vzh, double *vx, double *vy,
+              double *vz, double *pr, const TS *phi) {
   chain_begin();
   using V = typename Vec2<TS>::type;
   const int k0 = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
@@ -521,9 +521,9 @@ __global__ void __launch_bounds__(256)
     pjp2 = *reinterpret_cast<const V *>(phi + col_off(g, jp, i) + k0);
     pim2 = *reinterpret_cast<const V *>(phi + col_off(g, j, im) + k0);
     pip2 = *reinterpret_cast<const V *>(phi + col_off(g, j, ip) + k0);
-    uxh = __ldg(reinterpret_cast<const double2 *>(vxh + c + k0));
-    uyh = __ldg(reinterpret_cast<const double2 *>(vyh + c + k0));
-    uzh = __ldg(reinterpret_cast<const double2 *>(vzh + c + k0));
+    uxh = *reinterpret_cast<const double2 *>(vxh + c + k0);
+    uyh = *reinterpret_cast<const double2 *>(vyh + c + k0);
+    uzh = *reinterpret_cast<const double2 *>(vzh + c + k0);
     upr = *reinterpret_cast<const double2 *>(pr + c + k0);
   }
   // x-neighbours: phi(k0-1) is the left thread's second value, phi(k0+2) the right thread's
@@ -569,7 +569,7 @@ __global__ void __launch_bounds__(256)
     vz[c + k0] = oz.x;
     pr[c + k0] = op.x;
   }
-  if (k0 + 1 >= nxm - 1) vx[c + nxm] = __ldg(vxh + c + nxm);  // the upper wall value is copied
+  if (k0 + 1 >= nxm - 1) vx[c + nxm] = vxh[c + nxm];  // the upper wall value is copied
 }
 
 // ------------------------------------------------------------------------------------------
@@ -589,8 +589,8 @@ __device__ __forceinline__ double warp_sum(double v) {
 
 template <bool DIV>
 __global__ void __launch_bounds__(256)
-    k_max_reduce(Geom g, Tables t, const double *__restrict__ vx, const double *__restrict__ vy,
-                 const double *__restrict__ vz, unsigned long long *__restrict__ out) {
+    k_max_reduce(Geom g, Tables t, const double *vx, const double *vy,
+                 const double *vz, unsigned long long *out) {
   chain_begin();
   __shared__ double red[8];
   double m = 0.0;
@@ -696,10 +696,10 @@ __device__ __forceinline__ int tsw(int r, int c) { return r * 8 + (c ^ zsw(r)); 
 // at one z index i.  The real tile is the complex tile read as (re, im) = (x point 2c, 2c+1).
 template <int N1, typename TS>
 __global__ void __launch_bounds__(256)
-    k_div_fft_y_w(Geom g0, Tables t, const StepCoef *__restrict__ sc_all, int ns,
-                  const double *__restrict__ vx, const double *__restrict__ vy,
-                  const double *__restrict__ vz, typename Cplx<TS>::type *__restrict__ spec,
-                  const typename Cplx<TS>::type *__restrict__ tw, const double *__restrict__ field) {
+    k_div_fft_y_w(Geom g0, Tables t, const StepCoef *sc_all, int ns,
+                  const double *vx, const double *vy,
+                  const double *vz, typename Cplx<TS>::type *spec,
+                  const typename Cplx<TS>::type *__restrict__ tw, const double *field) {
   chain_begin();
   using C = typename Cplx<TS>::type;
   constexpr int N = 32 * N1;
@@ -722,26 +722,26 @@ __global__ void __launch_bounds__(256)
   const int nxm = g.nxm;
   const double2 ux = (kk < nxm) ? __ldg(reinterpret_cast<const double2 *>(t.udx3m + kk)) : make_double2(0.0, 0.0);
   (void)Tr;
+  const int d2 = kk + 1 < nxm ? 2 : 1;  // an existing value where the pair's second point does not
 #pragma unroll 4
   for (int j = threadIdx.x >> 3; j < N; j += 32) {
     double dv0 = 0.0, dv1 = 0.0;
     if (kk < nxm && field) {  // spectra: the field itself
-      const double2 f = __ldg(reinterpret_cast<const double2 *>(field + col_off(g, j, i) + kk));
+      const double2 f = *reinterpret_cast<const double2 *>(field + col_off(g, j, i) + kk);
       dv0 = f.x;
       dv1 = (kk + 1 < nxm) ? f.y : 0.0;
     } else if (kk < nxm) {
       const int jp = wrap_inc(j, N);
       const size_t c = col_off(g, j, i), cjp = col_off(g, jp, i), cip = col_off(g, j, ip);
-      const double2 zi = __ldg(reinterpret_cast<const double2 *>(vz + cip + kk));
-      const double2 zc = __ldg(reinterpret_cast<const double2 *>(vz + c + kk));
-      const double2 yj = __ldg(reinterpret_cast<const double2 *>(vy + cjp + kk));
-      const double2 yc = __ldg(reinterpret_cast<const double2 *>(vy + c + kk));
-      const double2 xc = __ldg(reinterpret_cast<const double2 *>(vx + c + kk));
+      const double2 zi = *reinterpret_cast<const double2 *>(vz + cip + kk);
+      const double2 zc = *reinterpret_cast<const double2 *>(vz + c + kk);
+      const double2 yj = *reinterpret_cast<const double2 *>(vy + cjp + kk);
+      const double2 yc = *reinterpret_cast<const double2 *>(vy + c + kk);
+      const double2 xc = *reinterpret_cast<const double2 *>(vx + c + kk);
+      const double x2 = vx[c + kk + d2];
       dv0 = ((zi.x - zc.x) * g.dz + (yj.x - yc.x) * g.dy + (xc.y - xc.x) * ux.x) * usdtal;
-      if (kk + 1 < nxm) {
-        const double x2 = __ldg(vx + c + kk + 2);
-        dv1 = ((zi.y - zc.y) * g.dz + (yj.y - yc.y) * g.dy + (x2 - xc.y) * ux.y) * usdtal;
-      }
+      const double dv = ((zi.y - zc.y) * g.dz + (yj.y - yc.y) * g.dy + (x2 - xc.y) * ux.y) * usdtal;
+      dv1 = d2 == 2 ? dv : 0.0;
     }
     C z;
     z.x = (TS)dv0;
@@ -851,8 +851,8 @@ __host__ __device__ constexpr int div_nbuf() {
 
 template <int N1>
 __global__ void __launch_bounds__(256, div_blocks_by_regs<N1>())
-    k_div_fft_y_wt(Geom g, Tables t, const StepCoef *__restrict__ sc_all, int ns, const __grid_constant__ DivMaps mp,
-                   double2 *__restrict__ spec, const double2 *__restrict__ tw, int *__restrict__ err) {
+    k_div_fft_y_wt(Geom g, Tables t, const StepCoef *sc_all, int ns, const __grid_constant__ DivMaps mp,
+                   double2 *spec, const double2 *__restrict__ tw, int *err) {
   chain_begin();
   constexpr int N = 32 * N1;
   if (!inst_active(g, 0)) return;  // a single domain stopped by its step control
@@ -975,7 +975,7 @@ __global__ void __launch_bounds__(256, div_blocks_by_regs<N1>())
 // K3w / K5w: z c2c in place.  Block: 8 x points (8 warps) at one ky.
 template <int N1, bool INV, typename TS>
 __global__ void __launch_bounds__(256)
-    k_fft_z_w(Geom g, typename Cplx<TS>::type *__restrict__ spec,
+    k_fft_z_w(Geom g, typename Cplx<TS>::type *spec,
               const typename Cplx<TS>::type *__restrict__ tw) {
   chain_begin();
   using C = typename Cplx<TS>::type;
@@ -1033,7 +1033,7 @@ __global__ void __launch_bounds__(256)
 // are in flight while the current tile is transformed and stored.  Same arithmetic as k_fft_z_w.
 template <int N1, bool INV, typename TS>
 __global__ void __launch_bounds__(256)
-    k_fft_z_wp(Geom g, typename Cplx<TS>::type *__restrict__ spec,
+    k_fft_z_wp(Geom g, typename Cplx<TS>::type *spec,
                const typename Cplx<TS>::type *__restrict__ tw) {
   chain_begin();
   using C = typename Cplx<TS>::type;
@@ -1130,7 +1130,7 @@ __device__ __forceinline__ int zslot(int k1, int rl) {
 template <int N1, bool INV, typename TS>
 __global__ void __launch_bounds__(256)
     k_fft_z_wt(Geom g, const __grid_constant__ CUtensorMap ld_map, const __grid_constant__ CUtensorMap st_map,
-               const typename Cplx<TS>::type *__restrict__ tw, int *__restrict__ err) {
+               const typename Cplx<TS>::type *__restrict__ tw, int *err) {
   chain_begin();
   using C = typename Cplx<TS>::type;
   constexpr int N = 32 * N1;
@@ -1265,7 +1265,7 @@ static bool fftz_tmaps(const Geom &g, int N1, typename Cplx<TS>::type *spec, CUt
 // at once); each warp then builds its packed sequence straight from them.
 template <int N1, typename TS>
 __global__ void __launch_bounds__(256)
-    k_ifft_y_w(Geom g, const typename Cplx<TS>::type *__restrict__ spec, TS *__restrict__ phi,
+    k_ifft_y_w(Geom g, const typename Cplx<TS>::type *spec, TS *phi,
                const typename Cplx<TS>::type *__restrict__ tw) {
   chain_begin();
   using C = typename Cplx<TS>::type;
@@ -1350,7 +1350,7 @@ __global__ void __launch_bounds__(256)
 template <int N1>
 __global__ void __launch_bounds__(256)
     k_ifft_y_wt(Geom g, const __grid_constant__ CUtensorMap ld_map, const __grid_constant__ CUtensorMap st_map,
-                const double2 *__restrict__ tw, int *__restrict__ err) {
+                const double2 *__restrict__ tw, int *err) {
   chain_begin();
   constexpr int N = 32 * N1;
   constexpr int NH = N / 2 + 1;
@@ -1532,7 +1532,7 @@ cudaError_t launch_explicit_implicit(const LaunchCtx &L, const SubstepBuffers &b
 // ------------------------------------------------------------------------------------------
 template <int M, int WPB, typename TS>
 __global__ void __launch_bounds__(WPB * 32, (WPB == 4) ? 4 : 2)
-    k_tridiag_pressure_p(Geom g, Tables t, typename Cplx<TS>::type *__restrict__ spec, int *__restrict__ err) {
+    k_tridiag_pressure_p(Geom g, Tables t, typename Cplx<TS>::type *spec, int *err) {
   chain_begin();
   using C = typename Cplx<TS>::type;
   extern __shared__ double smem_k4p[];

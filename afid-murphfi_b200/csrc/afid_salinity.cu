@@ -36,22 +36,20 @@ __device__ __forceinline__ int wrapmod(int a, int n) {
 
 // Wall-extended coarse column (InterpVelMgrd.F90:40-41, 75-76, 107-108): row -1 is
 // (1 - 2 inslwS) row 0, row nxm is (1 - 2 inslwN) row nxm-1, rows -2 and nxm+1 are zero.
-__device__ __forceinline__ double coarse_ext(const double *__restrict__ col, int r, int nxm, double fs, double fn) {
-  if (r >= 0 && r < nxm) return __ldg(col + r);
-  if (r == -1) return fs * __ldg(col);
-  if (r == nxm) return fn * __ldg(col + nxm - 1);
-  return 0.0;
+__device__ __forceinline__ double coarse_ext(const double *col, int r, int nxm, double fs, double fn) {
+  const double c = gld(col + min(max(r, 0), nxm - 1));
+  return (r >= 0 && r < nxm) ? c : r == -1 ? fs * c : r == nxm ? fn * c : 0.0;
 }
 
 // Wall-extended refined salinity (salinity.F90:462-481): row -1 is 2 salbp - sal(0) with SfixS
 // (else sal(0)), row nxmr is 2 saltp - sal(nxmr-1) with SfixN (else sal(nxmr-1)); -2 and nxmr+1
 // are zero.
 // The plate values are read only for the ghost rows.
-__device__ __forceinline__ double sal_ext(const double *__restrict__ col, int r, int n, int sfixs, int sfixn,
-                                          const double *__restrict__ bp, const double *__restrict__ tp) {
-  if (r >= 0 && r < n) return __ldg(col + r);
-  if (r == -1) return sfixs ? 2.0 * __ldg(bp) - __ldg(col) : __ldg(col);
-  if (r == n) return sfixn ? 2.0 * __ldg(tp) - __ldg(col + n - 1) : __ldg(col + n - 1);
+__device__ __forceinline__ double sal_ext(double c, int r, int n, int sfixs, int sfixn, const double *bp,
+                                          const double *tp) {
+  if (r >= 0 && r < n) return c;
+  if (r == -1) return sfixs ? 2.0 * __ldg(bp) - c : c;
+  if (r == n) return sfixn ? 2.0 * __ldg(tp) - c : c;
   return 0.0;
 }
 
@@ -59,9 +57,9 @@ __device__ __forceinline__ double sal_ext(const double *__restrict__ col, int r,
 // k_sal_grad: one thread per coarse cell (k < nxm) of the padded field.
 // ------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256)
-    k_sal_grad(Geom g, Tables t, const double *__restrict__ vx, const double *__restrict__ vy,
-               const double *__restrict__ vz, double *__restrict__ gx, double *__restrict__ gy,
-               double *__restrict__ gz) {
+    k_sal_grad(Geom g, Tables t, const double *vx, const double *vy,
+               const double *vz, double *gx, double *gy,
+               double *gz) {
   chain_begin();
   const size_t n = (size_t)g.ldx * g.nym * g.nzm;
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
@@ -70,9 +68,11 @@ __global__ void __launch_bounds__(256)
     const size_t col = e / g.ldx;
     const int j = (int)(col % g.nym), i = (int)(col / g.nym);
     const size_t ojp = col_off(g, wrap_inc(j, g.nym), i) + k, oip = col_off(g, j, wrap_inc(i, g.nzm)) + k;
-    gx[e] = (vx[e + 1] - vx[e]) * __ldg(t.udx3m + k);  // InterpVelMgrd.F90:37
-    gy[e] = (vy[ojp] - vy[e]) * g.dy;                   // :72
-    gz[e] = (vz[oip] - vz[e]) * g.dz;                   // :156
+    const double x0 = gld(vx + e), x1 = gld(vx + e + 1), y0 = gld(vy + e), y1 = gld(vy + ojp);
+    const double z0 = gld(vz + e), z1 = gld(vz + oip);
+    gx[e] = (x1 - x0) * __ldg(t.udx3m + k);  // InterpVelMgrd.F90:37
+    gy[e] = (y1 - y0) * g.dy;                // :72
+    gz[e] = (z1 - z0) * g.dz;                // :156
   }
 }
 
@@ -87,8 +87,8 @@ __global__ void __launch_bounds__(256)
 //                for the y and z integrations.
 // ------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(128)
-    k_sal_zint(Geom g, SalGeom sg, SalTables st, const double *__restrict__ gx, const double *__restrict__ gy,
-               const double *__restrict__ gz, double *__restrict__ tz) {
+    k_sal_zint(Geom g, SalGeom sg, SalTables st, const double *gx, const double *gy,
+               const double *gz, double *tz) {
   chain_begin();
   // block per output column (jc, ir): the four source columns and weights are block constants
   const int jc = blockIdx.x % g.nym, ir = blockIdx.x / g.nym;
@@ -104,10 +104,14 @@ __global__ void __launch_bounds__(128)
   }
   const double *src[3] = {gx, gy, gz};
   for (int r = threadIdx.x; r < g.nxm; r += blockDim.x) {
+    double e[3][4];
 #pragma unroll
     for (int f = 0; f < 3; ++f)
-      tz[(size_t)f * n + out + r] = __ldg(src[f] + o[0] + r) * w[0] + __ldg(src[f] + o[1] + r) * w[1] +
-                                    __ldg(src[f] + o[2] + r) * w[2] + __ldg(src[f] + o[3] + r) * w[3];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) e[f][c] = gld(src[f] + o[c] + r);
+#pragma unroll
+    for (int f = 0; f < 3; ++f)
+      tz[(size_t)f * n + out + r] = e[f][0] * w[0] + e[f][1] * w[1] + e[f][2] * w[2] + e[f][3] * w[3];
   }
 }
 
@@ -117,8 +121,8 @@ __global__ void __launch_bounds__(128)
 constexpr int kToRefWarps = 4;
 
 __global__ void __launch_bounds__(32 * kToRefWarps)
-    k_sal_to_ref(Geom g, SalGeom sg, SalTables st, const double *__restrict__ tz, double *__restrict__ vxr,
-                 double *__restrict__ gyr, double *__restrict__ gzr) {
+    k_sal_to_ref(Geom g, SalGeom sg, SalTables st, const double *tz, double *vxr,
+                 double *gyr, double *gzr) {
   chain_begin();
   extern __shared__ __align__(16) double sm_to_ref[];
   const int nxm = g.nxm, L = nxm + 4;  // extended rows -2 .. nxm+1 at 0 .. nxm+3
@@ -141,7 +145,7 @@ __global__ void __launch_bounds__(32 * kToRefWarps)
 #pragma unroll
     for (int f = 0; f < 3; ++f) {
       const double *t = tz + (size_t)f * n + r;
-      q[f] = __ldg(t + co[0]) * wy[0] + __ldg(t + co[1]) * wy[1] + __ldg(t + co[2]) * wy[2] + __ldg(t + co[3]) * wy[3];
+      q[f] = t[co[0]] * wy[0] + t[co[1]] * wy[1] + t[co[2]] * wy[2] + t[co[3]] * wy[3];
     }
     qx[r + 2] = q[0];
     qy[r + 2] = q[1];
@@ -185,14 +189,39 @@ __global__ void __launch_bounds__(32 * kToRefWarps)
   }
 }
 
+// out[m stride] = v + l (grad[0] + .. + grad[(m - 1) stride]), m = 1 .. n - 1, summed in order.  A load
+// may not pass the store of an earlier sum, so kScanAhead of them are issued before the stores (a
+// 6-step run with 384^3 refined cells: 49.4 ms with 16, 49.8 with 8, 49.6 with 4; 160 x 108 x 100
+// refined cells 4.28, 4.33, 4.48).
+constexpr int kScanAhead = 16;
+__device__ __forceinline__ void scan_line(const double *grad, double *out, size_t stride, int n, double v, double l) {
+  int m = 1;
+  for (; m + kScanAhead <= n; m += kScanAhead) {
+    double d[kScanAhead];
+#pragma unroll
+    for (int q = 0; q < kScanAhead; ++q, grad += stride) d[q] = gld(grad);
+#pragma unroll
+    for (int q = 0; q < kScanAhead; ++q) {
+      v = v + d[q] * l;
+      out += stride;
+      *out = v;
+    }
+  }
+  for (; m < n; ++m, grad += stride) {
+    v = v + gld(grad) * l;
+    out += stride;
+    *out = v;
+  }
+}
+
 // ------------------------------------------------------------------------------------------
 // k_sal_scan_y: thread per (kr, ir).  vyr at the plane y = 0 (jcr0 = 1) is vy(:, 1, :)
 // interpolated in x-z (InterpVelMgrd.F90:99-116: z contracted first, then x); then
 // vyr(jr+1) = vyr(jr) + dvy/dy(jr) / dyr (:124-131).  One rank: the MPI_SCAN correction is zero.
 // ------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(128)
-    k_sal_scan_y(Geom g, SalGeom sg, SalTables st, const double *__restrict__ vy, const double *__restrict__ gyr,
-                 double *__restrict__ vyr) {
+    k_sal_scan_y(Geom g, SalGeom sg, SalTables st, const double *vy, const double *gyr,
+                 double *vyr) {
   chain_begin();
   const int kr = blockIdx.x * blockDim.x + threadIdx.x, ir = blockIdx.y;
   if (kr >= sg.nxmr) return;
@@ -211,13 +240,9 @@ __global__ void __launch_bounds__(128)
     const double e = q1 * __ldg(st.w[0] + 4 * kr + a);
     v = (a == 0) ? e : v + e;
   }
-  size_t o = (size_t)sg.nymr * ir * sg.ldr + kr;
+  const size_t o = (size_t)sg.nymr * ir * sg.ldr + kr;
   vyr[o] = v;
-  for (int jr = 0; jr + 1 < sg.nymr; ++jr) {
-    v = v + __ldg(gyr + o) * sg.lya;
-    o += sg.ldr;
-    vyr[o] = v;
-  }
+  scan_line(gyr + o, vyr + o, sg.ldr, sg.nymr, v, sg.lya);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -226,8 +251,8 @@ __global__ void __launch_bounds__(128)
 // reference's `ic0 < xend(3)`); then vzr(ir+1) = vzr(ir) + dvz/dz(ir) / dzr (:206-213).
 // ------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(128)
-    k_sal_scan_z(Geom g, SalGeom sg, SalTables st, const double *__restrict__ vz, const double *__restrict__ gzr,
-                 double *__restrict__ vzr) {
+    k_sal_scan_z(Geom g, SalGeom sg, SalTables st, const double *vz, const double *gzr,
+                 double *vzr) {
   chain_begin();
   const int kr = blockIdx.x * blockDim.x + threadIdx.x, jr = blockIdx.y;
   if (kr >= sg.nxmr) return;
@@ -249,13 +274,9 @@ __global__ void __launch_bounds__(128)
     }
   }
   const size_t plane = (size_t)sg.nymr * sg.ldr;
-  size_t o = (size_t)jr * sg.ldr + kr;
+  const size_t o = (size_t)jr * sg.ldr + kr;
   vzr[o] = v;
-  for (int ir = 0; ir + 1 < sg.nzmr; ++ir) {
-    v = v + __ldg(gzr + o) * sg.lza;
-    o += plane;
-    vzr[o] = v;
-  }
+  scan_line(gzr + o, vzr + o, plane, sg.nzmr, v, sg.lza);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -269,7 +290,7 @@ __global__ void __launch_bounds__(128)
 //                    in shared memory, then salc(k) = sum_a wx_a(k) U2(sx(k) + a).
 // ------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(128)
-    k_sal_zc(Geom g, SalGeom sg, SalTables st, const double *__restrict__ sal, double *__restrict__ u) {
+    k_sal_zc(Geom g, SalGeom sg, SalTables st, const double *sal, double *u) {
   chain_begin();
   // block per output column (jr, ic): the four refined source columns, their plates and the
   // weights are block constants
@@ -287,10 +308,12 @@ __global__ void __launch_bounds__(128)
   double *out = u + ((size_t)jr + (size_t)sg.nymr * ic) * sg.ldu;
   for (int q = threadIdx.x; q < sg.nxmr + 4; q += blockDim.x) {
     const int rr = q - 2;
-    double v = 0.0;
+    double v = 0.0, row[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) row[c] = gld(colp[c] + min(max(rr, 0), sg.nxmr - 1));
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
-      const double s = sal_ext(colp[c], rr, sg.nxmr, sg.sfixs, sg.sfixn, st.salbp + pl[c], st.saltp + pl[c]) * w[c];
+      const double s = sal_ext(row[c], rr, sg.nxmr, sg.sfixs, sg.sfixn, st.salbp + pl[c], st.saltp + pl[c]) * w[c];
       v = (c == 0) ? s : v + s;
     }
     out[q] = v;
@@ -300,7 +323,7 @@ __global__ void __launch_bounds__(128)
 constexpr int kToCoarseWarps = 4;
 
 __global__ void __launch_bounds__(32 * kToCoarseWarps)
-    k_sal_to_coarse(Geom g, SalGeom sg, SalTables st, const double *__restrict__ u, double *__restrict__ salc) {
+    k_sal_to_coarse(Geom g, SalGeom sg, SalTables st, const double *u, double *salc) {
   chain_begin();
   // warp per coarse column (j, i), four per block, no block barriers
   extern __shared__ __align__(16) double sm_to_c[];
@@ -319,8 +342,8 @@ __global__ void __launch_bounds__(32 * kToCoarseWarps)
     co[b] = ((size_t)wrapmod(sy + b, sg.nymr) + (size_t)sg.nymr * i) * sg.ldu;
   }
   for (int r = lane; r < nrows; r += 32)
-    q[r] = __ldg(u + co[0] + r) * wy[0] + __ldg(u + co[1] + r) * wy[1] + __ldg(u + co[2] + r) * wy[2] +
-           __ldg(u + co[3] + r) * wy[3];
+    q[r] = u[co[0] + r] * wy[0] + u[co[1] + r] * wy[1] + u[co[2] + r] * wy[2] +
+           u[co[3] + r] * wy[3];
   __syncwarp();
   const size_t c0 = col_off(g, j, i);
   for (int k = lane; k < g.nxm; k += 32) {
@@ -342,10 +365,11 @@ __global__ void __launch_bounds__(32 * kToCoarseWarps)
 // are the column itself and those terms vanish; they are left out.
 //
 // Latency-bound: a column's loads wait for DRAM, then its solve is a serial chain, and other
-// resident columns hide both.  Five blocks per SM (at most 102 registers a thread) hide more of it
-// than the compiler's own choice at the price of 12 to 20 spilled bytes in 3-D, none in 2-D: 384^3
-// rows 1013 -> 883 us, 100 x 108 x 160 38.8 -> 34.5 us.  Six blocks spill 56 to 80 bytes from
-// MR = 4 on and measured 978 us; four give 1003 us.
+// resident columns hide both.  Five blocks per SM (96 registers a thread) hide more of it than the
+// compiler's own choice at the price of 24 to 36 spilled bytes in 3-D from MR = 4 on, none in 2-D:
+// 384^3 rows 1013 us a launch at the compiler's choice, 978 at six blocks, 1003 at four, 884 at
+// five; 791 with every load of a row batch, history and scaling included, ahead of its stores
+// (160 x 108 x 100 rows: 38 us).
 // ------------------------------------------------------------------------------------------
 constexpr int kSalStepWarps = 4;
 constexpr int kSalStepBlocks = 5;
@@ -357,9 +381,9 @@ __host__ __device__ inline size_t sal_step_smem(int MR, bool two_d) {
 
 template <int MR, bool TWO_D>
 __global__ void __launch_bounds__(32 * kSalStepWarps, kSalStepBlocks)
-    k_sal_step(SalGeom sg, SalTables st, const StepCoef *__restrict__ sc_all, int ns, const double *__restrict__ cn_tab,
-               const double *__restrict__ sal, const double *__restrict__ vxr, const double *__restrict__ vyr,
-               const double *__restrict__ vzr, double *__restrict__ rusal, double *__restrict__ sal_o) {
+    k_sal_step(SalGeom sg, SalTables st, const StepCoef *sc_all, int ns, const double *cn_tab,
+               const double *sal, const double *vxr, const double *vyr,
+               const double *vzr, double *rusal, double *sal_o) {
   chain_begin();
   constexpr int LD = chunk_ld(MR);
   constexpr int B = MR % 2 ? 1 : 2;  // rows per lane whose operands are loaded together
@@ -388,27 +412,28 @@ __global__ void __launch_bounds__(32 * kSalStepWarps, kSalStepBlocks)
     for (int q = 0; q < B; ++q) {
       const int k = lane + 32 * (p0 + q);
       const int kk = k < n ? k : n - 1;  // rows past the column read a valid row and are discarded
-      v[q][0] = __ldg(sal + c0 + kk);
-      v[q][1] = kk > 0 ? __ldg(sal + c0 + kk - 1) : 0.0;
-      v[q][2] = kk < n - 1 ? __ldg(sal + c0 + kk + 1) : 0.0;
-      v[q][3] = __ldg(sal + ojp + kk);
-      v[q][4] = __ldg(sal + ojm + kk);
-      v[q][5] = __ldg(vxr + c0 + kk);
-      v[q][6] = __ldg(vxr + c0 + kk + 1);
-      v[q][7] = __ldg(vyr + c0 + kk);
-      v[q][8] = __ldg(vyr + ojp + kk);
+      v[q][0] = gld(sal + c0 + kk);
+      v[q][1] = kk > 0 ? gld(sal + c0 + kk - 1) : 0.0;
+      v[q][2] = kk < n - 1 ? gld(sal + c0 + kk + 1) : 0.0;
+      v[q][3] = gld(sal + ojp + kk);
+      v[q][4] = gld(sal + ojm + kk);
+      v[q][5] = gld(vxr + c0 + kk);
+      v[q][6] = gld(vxr + c0 + kk + 1);
+      v[q][7] = gld(vyr + c0 + kk);
+      v[q][8] = gld(vyr + ojp + kk);
       if constexpr (!TWO_D) {
-        v[q][9] = __ldg(sal + oip + kk);
-        v[q][10] = __ldg(sal + oim + kk);
-        v[q][11] = __ldg(vzr + c0 + kk);
-        v[q][12] = __ldg(vzr + oip + kk);
+        v[q][9] = gld(sal + oip + kk);
+        v[q][10] = gld(sal + oim + kk);
+        v[q][11] = gld(vzr + c0 + kk);
+        v[q][12] = gld(vzr + oip + kk);
       }
     }
-    double ru[B];
+    double ru[B], tk[B];  // history and row scaling
 #pragma unroll
     for (int q = 0; q < B; ++q) {
       const int k = lane + 32 * (p0 + q);
-      ru[q] = rusal[c0 + (k < n ? k : n - 1)];
+      ru[q] = gld(rusal + c0 + (k < n ? k : n - 1));
+      tk[q] = gld(T + k);
     }
 #pragma unroll
     for (int q = 0; q < B; ++q) {
@@ -446,7 +471,7 @@ __global__ void __launch_bounds__(32 * kSalStepWarps, kSalStepBlocks)
           dxxs = sp * a_p + sc_ * a_c + sm * a_m;
         const double rhs = (sc.ga * hsal + sc.ro * ru[q] + alpec * dxxs) * sc.dt;
         rusal[c0 + k] = hsal;
-        rhs_s = rhs * __ldg(T + k);
+        rhs_s = rhs * tk[q];
       }
       s_rhs[(k % MR) * LD + k / MR] = rhs_s;
     }
@@ -454,10 +479,17 @@ __global__ void __launch_bounds__(32 * kSalStepWarps, kSalStepBlocks)
   __syncwarp();
   cn_solve_chunk<MR, LD>(s_rhs, T, lane);
   __syncwarp();
-#pragma unroll 4
-  for (int p = 0; p < MR; ++p) {
-    const int k = lane + 32 * p;
-    if (k < n) sal_o[c0 + k] = __ldg(sal + c0 + k) + s_rhs[(k % MR) * LD + k / MR];  // column re-read hits L1/L2
+  constexpr int U = MR % 4 == 0 ? 4 : MR % 3 == 0 ? 3 : MR;  // rows whose loads precede their stores
+#pragma unroll 1
+  for (int p = 0; p < MR; p += U) {
+    double c[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) c[u] = gld(sal + c0 + min(lane + 32 * (p + u), n - 1));  // re-read: L1/L2
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int k = lane + 32 * (p + u);
+      if (k < n) sal_o[c0 + k] = c[u] + s_rhs[(k % MR) * LD + k / MR];
+    }
   }
 }
 
@@ -483,8 +515,8 @@ cudaError_t launch_sal_step_M(const LaunchCtx &L, const SalCtx &S, int ns) {
 // CalcMaxCFL.F90:48-65: max over refined cells of |vz|/dz + |vy|/dy + |vx|/dx at the centre.
 // Non-negative doubles order like their bit patterns, so the maximum is an integer atomicMax.
 __global__ void __launch_bounds__(256)
-    k_sal_cfl(SalGeom sg, SalTables st, const double *__restrict__ vxr, const double *__restrict__ vyr,
-              const double *__restrict__ vzr, unsigned long long *__restrict__ out) {
+    k_sal_cfl(SalGeom sg, SalTables st, const double *vxr, const double *vyr,
+              const double *vzr, unsigned long long *out) {
   chain_begin();
   // blocks walk whole refined columns; a thread per row
   const int ncol = sg.nymr * sg.nzmr;
@@ -495,9 +527,9 @@ __global__ void __launch_bounds__(256)
     const size_t ojp = ((size_t)wrap_inc(j, sg.nymr) + (size_t)sg.nymr * i) * sg.ldr;
     const size_t oip = ((size_t)j + (size_t)sg.nymr * wrap_inc(i, sg.nzmr)) * sg.ldr;
     for (int k = threadIdx.x; k < sg.nxmr; k += blockDim.x) {
-      const double q = fabs((__ldg(vzr + o + k) + __ldg(vzr + oip + k)) * 0.5 * sg.dzr) +
-                       fabs((__ldg(vyr + o + k) + __ldg(vyr + ojp + k)) * 0.5 * sg.dyr) +
-                       fabs((__ldg(vxr + o + k) + __ldg(vxr + o + k + 1)) * 0.5 * __ldg(st.udx3mr + k));
+      const double q = fabs((vzr[o + k] + vzr[oip + k]) * 0.5 * sg.dzr) +
+                       fabs((vyr[o + k] + vyr[ojp + k]) * 0.5 * sg.dyr) +
+                       fabs((vxr[o + k] + vxr[o + k + 1]) * 0.5 * __ldg(st.udx3mr + k));
       m = nan_max(m, q);
     }
   }

@@ -12,6 +12,7 @@
 #include "afid_gpu.h"
 #include "afid_internal.h"
 #include "afid_salinity.h"
+#include "afid_tune.h"
 
 using namespace afid;
 
@@ -561,10 +562,13 @@ int ctx_run_substep(afid_ctx_t *ctx, int ns) { return run_substep(ctx, ns); }
 int ctx_fail(afid_ctx_t *ctx, cudaError_t e) { return fail_cuda(ctx, e); }
 
 // Time every K1 thread shape on the first `sample` columns and keep the fastest.  The RK3
-// histories all point at phi for these launches (K1 updates them in place; phi is dead between
-// substeps, as large as one history, and the values do not matter); the other outputs are
-// intermediates of the next substep or the idle temperature buffer, which the next K1 overwrites,
-// so the state is untouched.  Idle batch slots are timed as active.
+// histories, which K1 updates in place, are redirected for these launches to four places of their
+// own in phi and the spectrum (dead between substeps; the values do not matter) and, below about four
+// samples of columns, scratch memory: on one shared place the sample moved 88 bytes a cell of the
+// 136 in FP64 and ranked shapes by what it left out (512 x 512 x 384 mixed: a pick that takes 24.33 ms
+// a step against 24.01).  The other outputs are intermediates of the next substep or the idle
+// temperature buffer, which the next K1 overwrites, so the state is untouched.  Idle batch slots are
+// timed as active.
 int ctx_autotune(afid_ctx_t *ctx, bool force) {
   if (ctx->tuned && !force) return AFID_OK;
   LaunchCtx L = ctx->L;
@@ -587,7 +591,17 @@ int ctx_autotune(afid_ctx_t *ctx, bool force) {
   }
   if (n > 1) {
     SubstepBuffers b = buffers(ctx);
-    b.rux = b.ruy = b.ruz = b.rut = ctx->phi;
+    const size_t tsz = L.mixed ? sizeof(float) : sizeof(double);
+    const size_t dead[2] = {ctx->field_elems * tsz, (size_t)L.g.ldxc * L.g.nyh * L.g.nzm * 2 * tsz};
+    TunePlace place[4];
+    const size_t need = tune_places((size_t)sample * L.g.ldx * tsz, dead, place);
+    char *mem[3] = {static_cast<char *>(ctx->phi), static_cast<char *>(ctx->spec), nullptr};
+    if (need > 0 && cudaMalloc(&mem[2], need) != cudaSuccess) {
+      cudaGetLastError();  // no room: those histories share phi, the ranking is coarser
+      mem[2] = nullptr;
+    }
+    void **hist[4] = {&b.rux, &b.ruy, &b.ruz, &b.rut};
+    for (int q = 0; q < 4; ++q) *hist[q] = mem[place[q].mem] ? mem[place[q].mem] + place[q].offset : ctx->phi;
     L.g.active = nullptr;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     cudaError_t e = cudaEventCreate(&e0);
@@ -623,6 +637,8 @@ int ctx_autotune(afid_ctx_t *ctx, bool force) {
       }
     if (e0) cudaEventDestroy(e0);
     if (e1) cudaEventDestroy(e1);
+    const cudaError_t ef = cudaFree(mem[2]);
+    if (e == cudaSuccess) e = ef;
     if (e != cudaSuccess) return fail_cuda(ctx, e);
   }
   ctx->L.k1_var = info.chosen;

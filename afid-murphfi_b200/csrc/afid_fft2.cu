@@ -387,29 +387,29 @@ cudaError_t launch_r(const LaunchCtx &L, const SubstepBuffers &b, int ns, Stage 
   const int W = z ? 128 / (int)sizeof(C) : 8;
   const int threads = block_threads(W, std::max(f.r1, f.r2), THREE);
   const size_t smem = fft2_smem(f, W, sizeof(C), st);
-  auto fit = [&](auto kern) {
-    return smem > 48 * 1024 ? cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
-                            : cudaSuccess;
-  };
+  auto fit = [&](auto kern) { return smem > 48 * 1024 ? allow_dynamic_smem(kern) : cudaSuccess; };
   cudaError_t e;
   if (z) {
     const dim3 grid((g.nxm + W - 1) / W, g.nyh);
     auto kern = st == Stage::FftZFwd ? k_fft2_z<RMAX, THREE, false, TS> : k_fft2_z<RMAX, THREE, true, TS>;
     if ((e = fit(kern)) != cudaSuccess) return e;
-    return launch_chained(L, kern, grid, threads, smem, g, spec, f, twz);
+    launch_chained(L, kern, grid, threads, smem, g, spec, f, twz);
+    return cudaGetLastError();
   }
   const dim3 grid((g.nxm + 15) / 16, g.nzm);
   if constexpr (!THREE) {
     if (st == Stage::DivFftY) {
       auto kern = k_fft2_div<RMAX, TS>;
       if ((e = fit(kern)) != cudaSuccess) return e;
-      return launch_chained(L, kern, grid, threads, smem, g, L.t, b.sc, ns, b.vx_o, b.vy_o, b.vz_o, spec, f, twy,
-                            b.fft_field);
+      launch_chained(L, kern, grid, threads, smem, g, L.t, b.sc, ns, b.vx_o, b.vy_o, b.vz_o, spec, f, twy,
+                     b.fft_field);
+      return cudaGetLastError();
     }
   }
   auto kern = k_fft2_ify<RMAX, THREE, TS>;
   if ((e = fit(kern)) != cudaSuccess) return e;
-  return launch_chained(L, kern, grid, threads, smem, g, spec, (TS *)b.phi, f, twy);
+  launch_chained(L, kern, grid, threads, smem, g, spec, (TS *)b.phi, f, twy);
+  return cudaGetLastError();
 }
 
 }  // namespace
@@ -448,7 +448,7 @@ bool launch_fft2(const LaunchCtx &L, const SubstepBuffers &b, int ns, Stage st, 
   // The forward y transform by three gains nothing on k_div_fft_y, which is bound by the same loads of
   // the velocities (480 x 100 x 96 FP64 99 us against 84, 450 x 432 x 96 mixed 173 against 197).
   if (st == Stage::DivFftY && f.r3 > 1) return false;
-  if (fft2_smem(f, z ? 64 / (int)sizeof(TS) : 8, 2 * sizeof(TS), st) > (size_t)227 * 1024) return false;
+  if (fft2_smem(f, z ? 64 / (int)sizeof(TS) : 8, 2 * sizeof(TS), st) > kMaxDynSmem) return false;
   if (f.r3 > 1)
     *err = f.r1 <= 10 ? launch_r<10, true, TS>(L, b, ns, st, f) : launch_r<16, true, TS>(L, b, ns, st, f);
   else

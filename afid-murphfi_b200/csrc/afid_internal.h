@@ -62,6 +62,15 @@ inline cudaError_t launch_chained(const LaunchCtx &L, void (*kern)(P...), dim3 g
   return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
 }
 
+// Dynamic shared memory of the kernels whose need follows from a run-time length.  The limit belongs to
+// the kernel on the device, not to a context, so it is set to the most a block can have: a context on
+// another thread would otherwise lower it between this one's setting and its launch.
+constexpr size_t kMaxDynSmem = 227 * 1024;
+template <typename... P>
+inline cudaError_t allow_dynamic_smem(void (*kern)(P...)) {
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxDynSmem);
+}
+
 // Buffers of one substep.  K1 reads the state (vx, vy, vz, temp, pr) and writes the
 // intermediate fields (*_o); the pressure kernels read the intermediate velocities and write
 // the projected velocities back into the state arrays.

@@ -1932,15 +1932,15 @@ static cudaError_t launch_stage_T(const LaunchCtx &L, const SubstepBuffers &b, i
       const size_t smem = (size_t)TX * g.nym * sizeof(C);  // 2 buffers of TX/2 sequences
       dim3 grid((g.nxm + TX - 1) / TX, g.nzm);
       if (TX == 8) {
-        cudaFuncSetAttribute(k_div_fft_y<8, TS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        allow_dynamic_smem(k_div_fft_y<8, TS>);
         launch_chained(L, k_div_fft_y<8, TS>, grid, 256, smem, g, L.t, b.sc, ns, b.vx_o, b.vy_o, b.vz_o, spec,
                        L.plan_y, twy, b.fft_field);
       } else if (TX == 4) {
-        cudaFuncSetAttribute(k_div_fft_y<4, TS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        allow_dynamic_smem(k_div_fft_y<4, TS>);
         launch_chained(L, k_div_fft_y<4, TS>, grid, 256, smem, g, L.t, b.sc, ns, b.vx_o, b.vy_o, b.vz_o, spec,
                        L.plan_y, twy, b.fft_field);
       } else {
-        cudaFuncSetAttribute(k_div_fft_y<2, TS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        allow_dynamic_smem(k_div_fft_y<2, TS>);
         launch_chained(L, k_div_fft_y<2, TS>, grid, 256, smem, g, L.t, b.sc, ns, b.vx_o, b.vy_o, b.vz_o, spec,
                        L.plan_y, twy, b.fft_field);
       }
@@ -1955,7 +1955,7 @@ static cudaError_t launch_stage_T(const LaunchCtx &L, const SubstepBuffers &b, i
       const bool inv = (st == Stage::FftZInv);
 #define AFID_FFTZ(TXv, INVv)                                                                       \
   do {                                                                                             \
-    cudaFuncSetAttribute(k_fft_z<TXv, INVv, TS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+    allow_dynamic_smem(k_fft_z<TXv, INVv, TS>);                                                     \
     launch_chained(L, k_fft_z<TXv, INVv, TS>, grid, 256, smem, g, spec, L.plan_z, twz);                 \
   } while (0)
       if (TXZ == 8) { if (inv) AFID_FFTZ(8, true); else AFID_FFTZ(8, false); }
@@ -1972,13 +1972,13 @@ static cudaError_t launch_stage_T(const LaunchCtx &L, const SubstepBuffers &b, i
       dim3 grid((g.nxm + TX - 1) / TX, g.nzm);
       TS *phi = (TS *)b.phi;
       if (TX == 8) {
-        cudaFuncSetAttribute(k_ifft_y<8, TS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        allow_dynamic_smem(k_ifft_y<8, TS>);
         launch_chained(L, k_ifft_y<8, TS>, grid, 256, smem, g, spec, phi, L.plan_y, twy);
       } else if (TX == 4) {
-        cudaFuncSetAttribute(k_ifft_y<4, TS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        allow_dynamic_smem(k_ifft_y<4, TS>);
         launch_chained(L, k_ifft_y<4, TS>, grid, 256, smem, g, spec, phi, L.plan_y, twy);
       } else {
-        cudaFuncSetAttribute(k_ifft_y<2, TS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        allow_dynamic_smem(k_ifft_y<2, TS>);
         launch_chained(L, k_ifft_y<2, TS>, grid, 256, smem, g, spec, phi, L.plan_y, twy);
       }
       return cudaGetLastError();

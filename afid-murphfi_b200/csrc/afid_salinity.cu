@@ -641,7 +641,7 @@ cudaError_t launch_sal_interp(const LaunchCtx &L, const SalCtx &S, const double 
   launch_chained(L, k_sal_zint, g.nym * S.sg.nzmr, 128, 0, g, S.sg, S.st, S.gx, S.gy, S.gz, S.tmp);
   const size_t smem = (size_t)kToRefWarps * 3 * (g.nxm + 4) * sizeof(double);
   if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(k_sal_to_ref, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_dynamic_smem(k_sal_to_ref);
     if (e != cudaSuccess) return e;
   }
   const int ncr = S.sg.nymr * S.sg.nzmr;

@@ -1,16 +1,20 @@
 """The CFL and divergence maxima leave their accumulators ready for the next launch: calls in any
-order give the same values, and a divergence check between steps does not enter a batch's CFL."""
+order give the same values (the refined CFL's words lie beside theirs), and a divergence check
+before a step does not enter a batch's CFL."""
 import numpy as np
 import pytest
 
 import afid_gpu as ag
-from helpers import Case, bou_text
+from helpers import Case
 from oracle import afid_oracle as o
+from oracle import afid_salinity as sa
+from test_gpu_salinity import SalCase
 
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("shape", [(2, 6, 1), (33, 10, 6), (64, 96, 90)])  # one block .. more than 1184 columns
+@pytest.mark.parametrize("shape", [(2, 6, 1), (33, 10, 6), (64, 96, 90), (12, 120, 80)])
+# one block .. 1080 blocks of eight columns .. more columns than the largest grid's 1184 x 8 warps
 def test_maxima_repeat_in_any_order(shape):
     case = Case(*shape, rayt=1e6, dt=1e-3)
     s = case.oracle_state(random_velocity=0.3)
@@ -28,27 +32,40 @@ def test_maxima_repeat_in_any_order(shape):
         assert gpu.calc_max_cfl() == pytest.approx(0.25 * cfl, rel=1e-14)
 
 
+def test_maxima_of_both_grids_in_any_order():
+    c = SalCase((16, 16, 8), (24, 48, 32))  # 1536 refined columns for 1184 blocks
+    want = {"cfl": o.calc_max_cfl(c.g, c.s), "div": o.check_divergence(c.g, c.s),
+            "ref": sa.calc_max_cfl_refined(c.m, c.ss)}
+    assert len({round(v, 6) for v in want.values()}) == 3
+    with c.solver() as gpu:
+        call = {"cfl": gpu.calc_max_cfl, "div": gpu.check_divergence, "ref": gpu.sal_cfl}
+        for k in ("ref", "cfl", "ref", "ref", "div", "ref", "cfl", "div", "cfl", "ref"):
+            # the refined velocities are interpolated: the bound of tests/test_gpu_salinity.py
+            assert call[k]() == pytest.approx(want[k], rel=1e-12 if k == "ref" else 1e-14), k
+
+
 @pytest.mark.parametrize("nym,nzm,nslots", [(16, 1, 3), (50, 1, 2), (24, 16, 1)])  # one, several chunks; 3-D
-def test_divergence_check_between_batch_steps(nym, nzm, nslots):
-    inp = ag.parse_bou_in(bou_text(40, nym, nzm, rayt=1e6, idtv=1, dt=1e-3, cflmax=0.5, dtmax=5e-2))
-    rng = np.random.default_rng(3)
-
-    def make():
-        b = ag.Batch(inp, nslots)
-        for k in range(nslots):
-            f = [0.5 * rng_fields[q][k] for q in range(5)]
-            b.upload(k, *f)
-        b.set_active([1] * nslots)
-        return b
-
-    rng_fields = rng.standard_normal((5, nslots) + ((nzm, nym, 41) if nzm > 1 else (nym, 41)))
-    rng_fields[0, ..., 0] = rng_fields[0, ..., -1] = 0.0
-    with make() as a, make() as b:
-        for n in range(4):
-            a.step(1)
+def test_divergence_check_before_a_batch_step(nym, nzm, nslots):
+    """A field that alternates along y: its divergence is far above its CFL number, which averages
+    neighbours, so either one left in the other's place shows."""
+    dt = 1e-6
+    case = Case(40, nym, nzm, rayt=1e6, idtv=0, dt=dt, cflmax=1e3)
+    states = []
+    for k in range(nslots):
+        s = case.oracle_state(random_velocity=0.05, rng_seed=k)
+        s.vy[..., :40] += (5.0 + k) * (-1.0) ** np.arange(nym)[:, None]
+        states.append(s)
+    cfl = [o.calc_max_cfl(case.g, s) for s in states]
+    div = [o.check_divergence(case.g, s) for s in states]
+    assert all(d > 5 * c for c, d in zip(cfl, div))
+    with ag.Batch(case.inp, nslots) as b:
+        for check in (False, True, True):
+            for k, s in enumerate(states):
+                b.upload(k, s.vx, s.vy, s.vz, s.temp, s.pr)
+            b.set_active([1] * nslots)
+            if check:
+                # sums of a few terms in either order: rounding of the largest term
+                np.testing.assert_allclose(b.divmax(), div, rtol=1e-14)
             b.step(1)
-            if n != 2:
-                b.divmax()
-        sa, sb = a.stats(), b.stats()
-        for key in ("cfl", "dt", "time", "nu_vol"):
-            assert np.array_equal(sa[key], sb[key]), key
+            np.testing.assert_allclose(b.stats()["cfl"], np.array(cfl) * dt, rtol=1e-14)
+            assert b.divmax().max() < 1e-6 * min(div)  # projected

@@ -1,11 +1,14 @@
 """The wall-normal classes of 96 and 192 rows (three and six rows a lane of the partitioned solves) at
-their edges, against the oracle, and every launch shape of theirs against the first, bit for bit."""
+their edges, against the oracle, and every launch shape of theirs against the first, bit for bit; the same
+classes of the refined salinity rows."""
 import numpy as np
 import pytest
 
 import afid_gpu as ag
 from helpers import Case, rel_l2, rel_l2_mod_mean
 from oracle import afid_oracle as o
+from oracle import afid_salinity as sa
+from test_gpu_salinity import SalCase
 
 pytestmark = pytest.mark.gpu
 
@@ -54,3 +57,18 @@ def test_every_shape_bitwise_identical(shape, precision):
     for got in outs[1:]:
         for k in ag.Solver.FIELDS:
             assert np.array_equal(got[k], outs[0][k]), k
+
+
+@pytest.mark.parametrize("nxmr", [65, 96, 97, 129, 192])  # three and six refined rows a lane, and four and eight
+@pytest.mark.parametrize("nym,nzm", [(12, 6), (20, 1)])
+def test_refined_rows_at_class_edges(nxmr, nym, nzm):
+    c = SalCase((33, nym, nzm), (nxmr, 2 * nym, 2 * nzm if nzm > 1 else 1), istr3r=0)
+    with c.solver() as sv:
+        for n in range(2):
+            sv.time_marcher(1e-3, n)
+            sa.time_marcher(c.g, c.s, c.m, c.ss, 1e-3)
+        got, sal, salc = sv.download(), sv.sal_download(), sv.sal_aux()["salc"]
+    for f in ("vx", "vy", "vz", "temp"):  # the bound of tests/test_gpu_salinity.py
+        assert rel_l2(got[f], getattr(c.s, f)) < 1e-10, f
+    assert rel_l2(sal, c.ss.sal) < 1e-10
+    assert rel_l2(salc, c.ss.salc) < 1e-10

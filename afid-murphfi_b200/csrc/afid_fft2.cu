@@ -82,7 +82,6 @@ __device__ __forceinline__ void dft_any(int R, typename Cplx<T>::type (&x)[RMAX]
     case 16: dft_r<16, RMAX, INV, T>(x, tw, ts); break;
     case 18: dft_r<18, RMAX, INV, T>(x, tw, ts); break;
     case 20: dft_r<20, RMAX, INV, T>(x, tw, ts); break;
-    case 24: dft_r<24, RMAX, INV, T>(x, tw, ts); break;
     case 25: dft_r<25, RMAX, INV, T>(x, tw, ts); break;
   }
 }
@@ -415,11 +414,13 @@ cudaError_t launch_r(const LaunchCtx &L, const SubstepBuffers &b, int ns, Stage 
 }  // namespace
 
 // The factors of N: two up to 20 with the smaller larger one (r1 <= r2: more threads load, fewer values
-// each), else three up to 16, else two up to 25; r1 = 0 without any.  Above 20 the two transforms'
+// each), else three up to 16, else 625 = 25 x 25; r1 = 0 without any.  Above 20 the two transforms'
 // registers (180 to 255 in FP64) leave too few threads (1024 points by two transforms of 32, FP32: the
-// inverse y transform 36 us against 32 by three).
+// inverse y transform 36 us against 32 by three); every other length with such a factor splits
+// otherwise.  625 gains on the general kernels all the same: 64 x 625 x 64, z in FP64 33.1 -> 23.8
+// us, the y forward transform in mixed 53.7 -> 35.2 (in FP64 59.8 -> 64.8).
 FftSplit fft2_split(int N) {
-  static const int kR[] = {1, 2, 3, 4, 5, 6, 8, 9, 10, 12, 15, 16, 18, 20, 24, 25};
+  static const int kR[] = {1, 2, 3, 4, 5, 6, 8, 9, 10, 12, 15, 16, 18, 20, 25};
   FftSplit f{0, 0, 0, 0};
   int best = 1 << 30;
   auto take = [&](int a, int b, int c, int most, int rank) {
@@ -445,8 +446,9 @@ bool launch_fft2(const LaunchCtx &L, const SubstepBuffers &b, int ns, Stage st, 
   const bool z = st == Stage::FftZFwd || st == Stage::FftZInv;
   const Split f = z ? L.split_z : L.split_y;
   if (f.r1 == 0) return false;
-  // The forward y transform by three gains nothing on k_div_fft_y, which is bound by the same loads of
-  // the velocities (480 x 100 x 96 FP64 99 us against 84, 450 x 432 x 96 mixed 173 against 197).
+  // The forward y transform by three is not built: against k_div_fft_y, which is bound by the same loads
+  // of the velocities, it took 99 us and not 84 in FP64 (480 x 100 x 96); in mixed it would be the
+  // faster one (450 x 432 x 96: 173 and not 197).
   if (st == Stage::DivFftY && f.r3 > 1) return false;
   if (fft2_smem(f, z ? 64 / (int)sizeof(TS) : 8, 2 * sizeof(TS), st) > kMaxDynSmem) return false;
   if (f.r3 > 1)

@@ -37,6 +37,11 @@ __device__ __forceinline__ double gld(const double *p) {
   asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
   return v;
 }
+__device__ __forceinline__ double2 gld2(const double *p) {
+  double2 v;
+  asm volatile("ld.global.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p) : "memory");
+  return v;
+}
 constexpr int kMaxFftPasses = 24;
 
 struct Geom {

@@ -723,7 +723,9 @@ __global__ void __launch_bounds__(256)
   const double2 ux = (kk < nxm) ? __ldg(reinterpret_cast<const double2 *>(t.udx3m + kk)) : make_double2(0.0, 0.0);
   (void)Tr;
   const int d2 = kk + 1 < nxm ? 2 : 1;  // an existing value where the pair's second point does not
-#pragma unroll 4
+  // rows in flight a thread: two, one at 128 points (256 x N x 256 mixed, us a launch: N = 64 42.5 with
+  // four and 38.6, 128 74.2 and 71.9 (78.7 with two), 192 100.2 and 92.7, 256 129.3 and 117.4)
+#pragma unroll (N1 == 4 ? 1 : 2)
   for (int j = threadIdx.x >> 3; j < N; j += 32) {
     double dv0 = 0.0, dv1 = 0.0;
     if (kk < nxm && field) {  // spectra: the field itself
@@ -733,12 +735,12 @@ __global__ void __launch_bounds__(256)
     } else if (kk < nxm) {
       const int jp = wrap_inc(j, N);
       const size_t c = col_off(g, j, i), cjp = col_off(g, jp, i), cip = col_off(g, j, ip);
-      const double2 zi = *reinterpret_cast<const double2 *>(vz + cip + kk);
-      const double2 zc = *reinterpret_cast<const double2 *>(vz + c + kk);
-      const double2 yj = *reinterpret_cast<const double2 *>(vy + cjp + kk);
-      const double2 yc = *reinterpret_cast<const double2 *>(vy + c + kk);
-      const double2 xc = *reinterpret_cast<const double2 *>(vx + c + kk);
-      const double x2 = vx[c + kk + d2];
+      const double2 zi = gld2(vz + cip + kk);
+      const double2 zc = gld2(vz + c + kk);
+      const double2 yj = gld2(vy + cjp + kk);
+      const double2 yc = gld2(vy + c + kk);
+      const double2 xc = gld2(vx + c + kk);
+      const double x2 = gld(vx + c + kk + d2);
       dv0 = ((zi.x - zc.x) * g.dz + (yj.x - yc.x) * g.dy + (xc.y - xc.x) * ux.x) * usdtal;
       const double dv = ((zi.y - zc.y) * g.dz + (yj.y - yc.y) * g.dy + (x2 - xc.y) * ux.y) * usdtal;
       dv1 = d2 == 2 ? dv : 0.0;

@@ -577,10 +577,14 @@ int ctx_autotune(afid_ctx_t *ctx, bool force) {
   afid_tune_info_t info{};
   info.ncand = n;
   const int ncol = L.g.nym * L.g.nzm;
-  // 18 waves of one-column blocks at four a SM.  With a third of that, shapes of other blocks per SM
-  // were ranked by their last wave (240 x 200 x 180: a two-column shape 38.5 us a sample against
-  // 38.9, 537 us a launch against 487).
-  const int sample = std::min(ncol, 148 * 72);
+  // A whole number of waves for 2 to 6 one- or two-column blocks an SM, so that shapes are not ranked by
+  // their last wave (10656 columns: 256 x 256 x 250 mixed, a tie of shapes that take 739 and 725 us a
+  // launch), and more than twice the L2 cache (126 MB), so that the repeated launches come from memory
+  // as a large domain's do (10656 columns of 64 rows sit in it: 324 us a launch picked over 302).
+  constexpr int kWaves = 148 * 120;
+  const size_t tsz = L.mixed ? sizeof(float) : sizeof(double);
+  const size_t col_bytes = (size_t)L.g.ldx * (9 * sizeof(double) + 8 * tsz);  // nine fields, histories in and out
+  const int sample = std::min(ncol, kWaves * (1 + (int)(((size_t)256 << 20) / col_bytes / kWaves)));
   info.sample_columns = sample;
   for (int v = 0; v < AFID_TUNE_MAX; ++v) {
     info.threads[v] = v < n ? tpc[v] : 0;
@@ -591,7 +595,6 @@ int ctx_autotune(afid_ctx_t *ctx, bool force) {
   }
   if (n > 1) {
     SubstepBuffers b = buffers(ctx);
-    const size_t tsz = L.mixed ? sizeof(float) : sizeof(double);
     const size_t dead[2] = {ctx->field_elems * tsz, (size_t)L.g.ldxc * L.g.nyh * L.g.nzm * 2 * tsz};
     TunePlace place[4];
     const size_t need = tune_places((size_t)sample * L.g.ldx * tsz, dead, place);
@@ -607,7 +610,7 @@ int ctx_autotune(afid_ctx_t *ctx, bool force) {
     cudaError_t e = cudaEventCreate(&e0);
     if (e == cudaSuccess) e = cudaEventCreate(&e1);
     double best = 1e300;
-    constexpr int kReps = 2;
+    const int kReps = std::max(1, std::min(4, kWaves / sample));  // short launches: a few in a row
     // two rounds over all candidates, keeping each one's best: the first round also brings the
     // clocks up, which would otherwise bias against the first candidates
     for (int round = 0; round < 2 && e == cudaSuccess; ++round) {

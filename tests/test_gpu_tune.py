@@ -9,8 +9,10 @@ from helpers import Case
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("shape", [(40, 20, 12), (33, 128, 100), (36, 216, 200)])  # scratch for two or three .. none
-@pytest.mark.parametrize("precision", [ag.PREC_FP64, ag.PREC_MIXED])
+# scratch for two or three histories (fewer columns than a sample), for one, for none
+@pytest.mark.parametrize("shape,precision", [((40, 20, 12), ag.PREC_FP64), ((40, 20, 12), ag.PREC_MIXED),
+                                             ((33, 128, 100), ag.PREC_MIXED), ((128, 200, 180), ag.PREC_FP64),
+                                             ((112, 300, 240), ag.PREC_FP64)])
 def test_tuning_between_steps_changes_nothing(shape, precision):
     case = Case(*shape, precision=precision, rayt=1e6, dt=1e-4)
     s = case.oracle_state(random_velocity=0.1)

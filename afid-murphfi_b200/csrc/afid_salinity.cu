@@ -366,13 +366,18 @@ __global__ void __launch_bounds__(32 * kToCoarseWarps)
 //
 // Latency-bound: a column's loads wait for DRAM, then its solve is a serial chain, and other
 // resident columns hide both.  Five blocks per SM (96 registers a thread) hide more of it than the
-// compiler's own choice at the price of 24 to 36 spilled bytes in 3-D from MR = 4 on, none in 2-D:
-// 384^3 rows 1013 us a launch at the compiler's choice, 978 at six blocks, 1003 at four, 884 at
-// five; 791 with every load of a row batch, history and scaling included, ahead of its stores
-// (160 x 108 x 100 rows: 38 us).
+// compiler's own choice at the price of 24 to 36 spilled bytes in 3-D, none in 2-D: 384^3 rows 1013
+// us a launch at the compiler's choice, 978 at six blocks, 1003 at four, 884 at five; 791 with every
+// load of a row batch, history and scaling included, ahead of its stores (160 x 108 x 100 rows:
+// 39 us).  From 16 rows a lane on (34 KB of solves a block at 32) two rows in flight at five
+// blocks wait longer for their loads, at the same hit rates and bytes, and other splits measured best;
+// us a launch, two rows and five blocks against the choice below:
+// 192 x 192 x 512 312 and 298, 128 x 128 x 700 246 and 211, 128 x 128 x 1000 376 and 335.
 // ------------------------------------------------------------------------------------------
 constexpr int kSalStepWarps = 4;
-constexpr int kSalStepBlocks = 5;
+// Rows per lane whose operands are loaded together, and resident blocks per SM.
+__host__ __device__ constexpr int sal_step_rows(int MR) { return MR % 2 || MR == 16 || MR == 32 ? 1 : 2; }
+__host__ __device__ constexpr int sal_step_blocks(int MR) { return MR == 16 ? 6 : MR == 24 ? 4 : 5; }
 
 __host__ __device__ inline size_t sal_step_smem(int MR, bool two_d) {
   (void)two_d;
@@ -380,13 +385,13 @@ __host__ __device__ inline size_t sal_step_smem(int MR, bool two_d) {
 }
 
 template <int MR, bool TWO_D>
-__global__ void __launch_bounds__(32 * kSalStepWarps, kSalStepBlocks)
+__global__ void __launch_bounds__(32 * kSalStepWarps, sal_step_blocks(MR))
     k_sal_step(SalGeom sg, SalTables st, const StepCoef *sc_all, int ns, const double *cn_tab,
                const double *sal, const double *vxr, const double *vyr,
                const double *vzr, double *rusal, double *sal_o) {
   chain_begin();
   constexpr int LD = chunk_ld(MR);
-  constexpr int B = MR % 2 ? 1 : 2;  // rows per lane whose operands are loaded together
+  constexpr int B = sal_step_rows(MR);
   static_assert(MR % B == 0, "row batches must tile the column");
   extern __shared__ __align__(16) double smem_sal[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -479,7 +484,7 @@ __global__ void __launch_bounds__(32 * kSalStepWarps, kSalStepBlocks)
   __syncwarp();
   cn_solve_chunk<MR, LD>(s_rhs, T, lane);
   __syncwarp();
-  constexpr int U = MR % 4 == 0 ? 4 : MR % 3 == 0 ? 3 : MR;  // rows whose loads precede their stores
+  constexpr int U = MR == 32 ? 8 : MR % 4 == 0 ? 4 : MR % 3 == 0 ? 3 : MR;  // rows whose loads precede their stores
 #pragma unroll 1
   for (int p = 0; p < MR; p += U) {
     double c[U];

@@ -11,7 +11,8 @@
 // barrier per radix-2..5 factor with runtime radices and divisions) stay for lengths without such
 // factors.
 //   240 x 200 (y x z) x 180 FP64, us a launch: z 86 -> 30 (0.72 of the copy bandwidth), y forward with
-//   the divergence 124 -> 102, y inverse 84 -> 37; 320 x 300 x 225 mixed: 110 -> 42, 202 -> 177, 136 -> 64;
+//   the divergence 124 -> 102, y inverse 84 -> 37; 320 x 300 x 225 mixed: 110 -> 42, 202 -> 177 (8% less
+//   again with coherent loads), 136 -> 64;
 //   three transforms, 450 x 432 x 96 mixed: z 128 -> 50, y inverse 133 -> 74; 480 x 100 x 96 FP64: 52 -> 37.
 // Lengths 32 x {..} keep the warp transform, which is as fast or faster there (384 FP64 z 116 us against
 // 203 by two transforms; 128 FP64 y forward 5.8 against 8.0).

@@ -39,12 +39,16 @@ struct LaunchCtx {
 
 // Launch of a kernel whose first statement is chain_begin(): the stream's order is kept by that
 // statement instead of by the launch, so the launch latencies of dependent kernels overlap with the
-// kernels before them.  Small domains are bound by them: a main-loop step of 128 x 64 cells (16
-// kernels) takes 62 us instead of 73, one of 47 x 60 x 50 90 instead of 105.  Not in a captured
-// step (L.chained off), where the programmatic edges cost more than plain ones: 25 steps of 24
-// 128 x 64 instances 4.00 ms against 3.87.  And not above kChainBlocks blocks, where the latency does
-// not count and the order in which waiting blocks are handed to the SMs does: 6 steps with 384^3
-// refined cells took 57 ms chained throughout and 53.7 with this limit or unchained.
+// kernels before them.  Small domains are bound by them: a main-loop step of 128 x 64 cells (17
+// kernels) takes 94 us instead of 120 on a slow host and 62 instead of 73 on a fast one, one of
+// 47 x 60 x 50 155 instead of 193.  Not in a batch (L.chained off), whose steps run captured, where
+// the programmatic edges cost more than plain ones: 25 steps of 24 128 x 64 instances 4.00 ms against
+// 3.87.  And not above kChainBlocks blocks, where the latency does not count and the order in which
+// waiting blocks are handed to the SMs does: 6 steps with 384^3 refined cells take 60.4 ms chained
+// throughout, 49.4 with this limit and 49.2 unchained; 512 x 512 x 384 mixed 26.6, 24.1 and 24.1 a
+// step.  Persistent kernels and the maxima stay below the limit at every size and are chained on the
+// largest domains too: 240 x 200 x 180 2595 us with this limit, 2622 unchained, 320 x 300 x 225 mixed
+// 5342 and 5330.
 constexpr size_t kChainBlocks = 148 * 32;
 template <typename... P, typename... A>
 inline cudaError_t launch_chained(const LaunchCtx &L, void (*kern)(P...), dim3 grid, dim3 block, size_t smem,

@@ -162,8 +162,8 @@ int afid_gpu_mean_plane(afid_ctx_t *ctx, int which, int axis, double *out);
  * per block)
  * is timed on a sample of columns, with the RK3 histories redirected to memory that is dead
  * between substeps (and scratch where that is too little) so the state is untouched, and the
- * fastest is kept.  It runs by itself before the first step; force = 1 repeats it.  The shape changes the schedule only: results are bitwise the same for
- * every shape. */
+ * fastest is kept.  It runs by itself before the first step; force = 1 repeats it.  The shape
+ * changes the schedule only: results are bitwise the same for every shape. */
 #define AFID_TUNE_MAX 8
 typedef struct afid_tune_info {
   int ncand;                    /* shapes available (1 = nothing to choose)                  */

@@ -723,9 +723,10 @@ __global__ void __launch_bounds__(256)
   const double2 ux = (kk < nxm) ? __ldg(reinterpret_cast<const double2 *>(t.udx3m + kk)) : make_double2(0.0, 0.0);
   (void)Tr;
   const int d2 = kk + 1 < nxm ? 2 : 1;  // an existing value where the pair's second point does not
-  // rows in flight a thread: two, one at 128 points (256 x N x 256 mixed, us a launch: N = 64 42.5 with
-  // four and 38.6, 128 74.2 and 71.9 (78.7 with two), 192 100.2 and 92.7, 256 129.3 and 117.4)
-#pragma unroll (N1 == 4 ? 1 : 2)
+  // rows in flight a thread: two, one at 128 points in FP32 (us a launch: 256 x N x 256 mixed N = 64 42.5
+  // with four and 38.6, 128 74.2 with four, 78.7 with two and 71.9, 192 100.2 and 92.7, 256 129.3 and
+  // 117.4; 24 instances of 64 x 128, less than a wave, FP64 6.64 with four, 6.80 with one and 5.66)
+#pragma unroll (N1 == 4 && sizeof(TS) == 4 ? 1 : 2)
   for (int j = threadIdx.x >> 3; j < N; j += 32) {
     double dv0 = 0.0, dv1 = 0.0;
     if (kk < nxm && field) {  // spectra: the field itself

@@ -610,7 +610,8 @@ int ctx_autotune(afid_ctx_t *ctx, bool force) {
     cudaError_t e = cudaEventCreate(&e0);
     if (e == cudaSuccess) e = cudaEventCreate(&e1);
     double best = 1e300;
-    const int kReps = std::max(1, std::min(4, kWaves / sample));  // short launches: a few in a row
+    // short launches several in a row: the timestamps of events step by about a microsecond
+    const int kReps = std::max(1, std::min(12, kWaves / sample));
     // two rounds over all candidates, keeping each one's best: the first round also brings the
     // clocks up, which would otherwise bias against the first candidates
     for (int round = 0; round < 2 && e == cudaSuccess; ++round) {
